@@ -83,7 +83,7 @@ typedef struct {
  * tsvd_set_frpca_seed() (the reference seeds MKL VSL with time(NULL)). The
  * caller's double values are rounded to float and both products run as FP32
  * SpMM on the GPU (tsvd_frpca_fp32); the small solves are fp32 with fp64
- * Grams and an fp64-refined eigen-solve, so results match the reference's
+ * Grams and an accurate eigen-solve, so results match the reference's
  * FP64 frPCA to about 1e-6 relative in the leading singular values, not to
  * double precision.
  * Errors are reported through tsvd_last_error(); the legacy signature has no
@@ -302,8 +302,7 @@ typedef struct tsvd_step_stats {
   int32_t eig_sweeps_merge; /* Jacobi sweeps of the merges (max over levels)      */
   int32_t merge_subspace_iters; /* subspace iterations of merges wider than 256  */
                             /* columns (max over levels; 0 for narrow merges)    */
-  int32_t eig_refine_sweeps;/* sweeps of the fp64 refinement Jacobi (max, all     */
-                            /* eigen-solves of the snapshot)                     */
+  int32_t eig_refine_sweeps;/* 0: a snapshot's eigen-solves have no second pass   */
   int32_t sparse_blocks;    /* blocks factorized through FP32 CSR SpMM            */
   double tune_density;      /* TSVD_BLOCKS_AUTO: density below which a block takes */
                             /* the SpMM path (0 before the first factorization)  */

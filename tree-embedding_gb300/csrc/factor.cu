@@ -12,7 +12,7 @@
 //
 // The merge follows Code/Tree_u_NC.cpp:723-850: M = [B_1 ... B_h], the
 // truncated SVD of M (dgesvd, ..._mkl.c:1259-1300) keeps U_d S_d; here the
-// Gram M^T M is diagonalized by Jacobi and B_parent = M V_d (= U_d S_d); the
+// Gram M^T M is diagonalized (eig.cu) and B_parent = M V_d (= U_d S_d); the
 // root keeps U sqrt(S) = M V_d S^-1/2 (NC) or U = M V_d S^-1 (LP).
 #include <algorithm>
 #include <cmath>
@@ -179,8 +179,10 @@ __global__ void lp_split_kernel(const float *__restrict__ u, int nsrc, int d, in
 
 }  // namespace
 
-tsvd_status frpca_work_alloc(FrpcaWork &W, int nmax, int64_t rows_max, int sp, int l, int d) {
+tsvd_status frpca_work_alloc(FrpcaWork &W, int nmax, int64_t rows_max, int sp, int l, int d,
+                             bool direct) {
   W.nmax = nmax;
+  W.direct = direct;
   W.rows_max = std::max<int64_t>(rows_max, 1);
   W.sp = sp;
   W.l = l;
@@ -206,8 +208,20 @@ tsvd_status frpca_work_alloc(FrpcaWork &W, int nmax, int64_t rows_max, int sp, i
     W.gram_bytes = (size_t)chunks * 256 * 256 * sizeof(double);
   }
   TSVD_CUDA(cudaMalloc(&W.gram_work, W.gram_bytes));
-  W.jac_bytes = std::max(jacobi_work_bytes(256, nmax), jacobi_work_bytes(l, nmax));
-  TSVD_CUDA(cudaMalloc(&W.jac_work, W.jac_bytes));
+  W.eig_bytes = eig_work_bytes(256, nmax);
+  TSVD_CUDA(cudaMalloc(&W.eig_work, W.eig_bytes));
+  TSVD_CUDA(cudaMalloc(&W.eig_stat, sizeof(int32_t)));
+  TSVD_CUDA(cudaMemset(W.eig_stat, 0, sizeof(int32_t)));
+  if (direct) {
+    W.jac_bytes = std::max(jacobi_work_bytes(256, nmax), jacobi_work_bytes(l, nmax));
+    TSVD_CUDA(cudaMalloc(&W.jac_work, W.jac_bytes));
+    for (double **p : {&W.dv, &W.dt, &W.dh})
+      TSVD_CUDA(cudaMalloc(p, (size_t)nmax * 256 * 256 * sizeof(double)));
+    std::vector<double *> hp(nmax);
+    for (int i = 0; i < nmax; ++i) hp[i] = W.dh + (int64_t)i * 256 * 256;
+    TSVD_CUDA(cudaMalloc(&W.dh_ptrs, sizeof(double *) * nmax));
+    TSVD_CUDA(cudaMemcpy(W.dh_ptrs, hp.data(), sizeof(double *) * nmax, cudaMemcpyHostToDevice));
+  }
   W.ptr_slots = (size_t)nmax * 64 + 256;
   TSVD_CUDA(cudaMalloc(&W.dptr, W.ptr_slots * sizeof(void *)));
   TSVD_CUDA(cudaMallocHost(&W.hptr, W.ptr_slots * sizeof(void *)));
@@ -216,28 +230,28 @@ tsvd_status frpca_work_alloc(FrpcaWork &W, int nmax, int64_t rows_max, int sp, i
   W.tmap_slots = (size_t)nmax * 6;
   TSVD_CUDA(cudaMalloc(&W.tmap_dev, W.tmap_slots * sizeof(CUtensorMap)));
   TSVD_CUDA(cudaMallocHost(&W.tmap_host, W.tmap_slots * sizeof(CUtensorMap)));
-  for (double **p : {&W.dv, &W.dt, &W.dh})
-    TSVD_CUDA(cudaMalloc(p, (size_t)nmax * 256 * 256 * sizeof(double)));
-  {
-    std::vector<double *> hp(nmax);
-    for (int i = 0; i < nmax; ++i) hp[i] = W.dh + (int64_t)i * 256 * 256;
-    TSVD_CUDA(cudaMalloc(&W.dh_ptrs, sizeof(double *) * nmax));
-    TSVD_CUDA(cudaMemcpy(W.dh_ptrs, hp.data(), sizeof(double *) * nmax, cudaMemcpyHostToDevice));
-  }
   return TSVD_OK;
 }
 
 void frpca_work_free(FrpcaWork &W) {
   cudaFree(W.xhi); cudaFree(W.xlo); cudaFree(W.z); cudaFree(W.y); cudaFree(W.qhi);
   cudaFree(W.qlo); cudaFree(W.g); cudaFree(W.t); cudaFree(W.lambda); cudaFree(W.v);
-  cudaFree(W.colscale); cudaFree(W.sums); cudaFree(W.gram_work); cudaFree(W.jac_work); cudaFree(W.dptr);
+  cudaFree(W.colscale); cudaFree(W.sums); cudaFree(W.gram_work); cudaFree(W.eig_work); cudaFree(W.eig_stat); cudaFree(W.dptr);
   cudaFreeHost(W.hptr); cudaFree(W.dint); cudaFreeHost(W.hint);
   cudaFree(W.tmap_dev); cudaFreeHost(W.tmap_host);
   cudaFree(W.wm); cudaFree(W.wv); cudaFree(W.ww); cudaFree(W.wy); cudaFree(W.wy2);
   cudaFree(W.wchol); cudaFree(W.wnorm); cudaFree(W.wk);
-  cudaFree(W.dv); cudaFree(W.dt); cudaFree(W.dh); cudaFree(W.dh_ptrs);
+  cudaFree(W.jac_work); cudaFree(W.dv); cudaFree(W.dt); cudaFree(W.dh); cudaFree(W.dh_ptrs);
   cudaGetLastError();  // the launch checks read this slot: leave nothing from teardown in it
   W = FrpcaWork();
+}
+
+// The largest sweep count of the eigen-solves since the last call, into
+// W.last_sweeps once st has been synchronized.
+tsvd_status eig_sweeps_fetch(FrpcaWork &W, cudaStream_t st) {
+  TSVD_CUDA(cudaMemcpyAsync(&W.last_sweeps, W.eig_stat, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  TSVD_CUDA(cudaMemsetAsync(W.eig_stat, 0, sizeof(int32_t), st));
+  return TSVD_OK;
 }
 
 namespace {
@@ -285,10 +299,10 @@ __global__ void __launch_bounds__(256) dgemm_small_kernel(const double *__restri
 // (W.v) are refined: H = V^T G V in fp64 (nearly diagonal), a Jacobi on H
 // that carries the diagonal in fp64, its rotations replayed onto V. lam / v:
 // pointer arrays to W.lambda / W.v of each problem.
-tsvd_status eig_refined(FrpcaWork &W, double *const *d_g, int n, float *const *d_lam,
+static tsvd_status eig_refined(FrpcaWork &W, double *const *d_g, int n, float *const *d_lam,
                         float *const *d_v, int nprob, cudaStream_t st) {
   TSVD_TRY(jacobi_eig_batched(d_g, n, d_lam, d_v, nprob, W.jac_work, W.jac_bytes, st,
-                              &W.last_sweeps));
+                              W.eig_stat));
   const int64_t S = 256 * 256;
   widen_kernel<<<dim3(grid_for((int64_t)n * n, 256, 1), nprob), 256, 0, st>>>(W.v, W.dv,
                                                                             (int64_t)n * n, S, S);
@@ -302,7 +316,15 @@ tsvd_status eig_refined(FrpcaWork &W, double *const *d_g, int n, float *const *d
   // the rotations are replayed onto V in place (each replay block reads its
   // rows before writing them)
   return jacobi_eig_batched(W.dh_ptrs, n, d_lam, d_v, nprob, W.jac_work, W.jac_bytes, st,
-                            &W.last_refine_sweeps, 1, (const float *const *)d_v);
+                            W.eig_stat, 1, (const float *const *)d_v);
+}
+
+// Eigenpairs of the Grams W.g (the nv leading eigenvectors): lam / v point into
+// W.lambda / W.v.
+static tsvd_status eig_solve(FrpcaWork &W, double *const *d_g, int n, int nv, float *const *d_lam,
+                             float *const *d_v, int nprob, cudaStream_t st) {
+  if (W.direct && n > kDirectOneSided) return eig_refined(W, d_g, n, d_lam, d_v, nprob, st);
+  return eig_gram_batched(d_g, n, nv, d_lam, d_v, nprob, W.eig_work, W.eig_bytes, W.eig_stat, st);
 }
 
 tsvd_status frpca_batch(FrpcaWork &W, const FrpcaProblem *probs, int nprob, int q, uint64_t seed,
@@ -439,7 +461,7 @@ tsvd_status frpca_batch(FrpcaWork &W, const FrpcaProblem *probs, int nprob, int 
   // eigSVD of Z = A^T Q (frpca.c:99-136): Gram, eigenpairs, top-d.
   TSVD_TRY(gram_batched((const float *const *)d_z, d_nc, max_nc, l, kLp, d_g, W.gram_work,
                         W.gram_bytes, nprob, st));
-  TSVD_TRY(eig_refined(W, d_g, l, d_lam, d_v, nprob, st));
+  TSVD_TRY(eig_solve(W, d_g, l, d, d_lam, d_v, nprob, st));
   double *d_sum2 = W.sums;
   sigma_kernel<<<nprob, 128, 0, st>>>((const float *const *)d_lam, d, d_cs, d_csi, d_sout, d_sum2);
   TSVD_LAUNCH_CHECK();
@@ -460,6 +482,7 @@ tsvd_status frpca_batch(FrpcaWork &W, const FrpcaProblem *probs, int nprob, int 
   }
   std::vector<double> hs(nprob);
   TSVD_CUDA(cudaMemcpyAsync(hs.data(), d_sum2, sizeof(double) * nprob, cudaMemcpyDeviceToHost, st));
+  TSVD_TRY(eig_sweeps_fetch(W, st));
   TSVD_CUDA(cudaStreamSynchronize(st));
   if (sum_sigma2)
     for (int i = 0; i < nprob; ++i) sum_sigma2[i] = hs[i];
@@ -469,7 +492,7 @@ tsvd_status frpca_batch(FrpcaWork &W, const FrpcaProblem *probs, int nprob, int 
 namespace {
 
 // The Rayleigh-Ritz end of a merge: for each problem, the n-column matrix
-// m[i] (|S| x n, ld n) -> Gram (compensated, fp64) -> Jacobi eigenpairs ->
+// m[i] (|S| x n, ld n) -> Gram (compensated, fp64) -> eigenpairs ->
 // out = m V_d diag(f(s)), sigma_out = s (the d largest singular values).
 tsvd_status merge_finish(FrpcaWork &W, const MergeProblem *probs, int nprob, int n, int nsrc,
                          int root_mode, const std::vector<float *> &m, cudaStream_t st) {
@@ -495,7 +518,7 @@ tsvd_status merge_finish(FrpcaWork &W, const MergeProblem *probs, int nprob, int
   TSVD_TRY(pk.upload(st));
   TSVD_TRY(gram_batched((const float *const *)d_m, d_rows, nsrc, n, n, d_g, W.gram_work,
                         W.gram_bytes, nprob, st));
-  TSVD_TRY(eig_refined(W, d_g, n, d_lam, d_v, nprob, st));
+  TSVD_TRY(eig_solve(W, d_g, n, d, d_lam, d_v, nprob, st));
   merge_scale_kernel<<<nprob, 128, 0, st>>>((const float *const *)d_lam, d, root_mode, d_cs,
                                             d_sout);
   TSVD_LAUNCH_CHECK();
@@ -605,7 +628,7 @@ tsvd_status orthonormalize(FrpcaWork &W, float *x, int64_t xstride, float *y, in
 // (Y = M V, W = M^T Y, each product re-orthonormalized by CholeskyQR on a
 // compensated Gram), started from the p columns of M with the largest norms
 // and stopped when ||M V||_F^2 gains less than 1e-7 of itself. The result is
-// then the merge of the p columns of M V (compensated Gram + Jacobi), the
+// then the merge of the p columns of M V (compensated Gram + eigen-solve), the
 // same arithmetic as a narrow merge. The products are plain fp32 GEMMs
 // (sgemm_batched: fixed-order sums, 64 x 64 tiles).
 tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, int n, int nsrc,

@@ -20,8 +20,14 @@ struct FrpcaWork {
   double *sums = nullptr;                  // [nmax] sum of kept sigma^2
   double *gram_work = nullptr;
   size_t gram_bytes = 0;
-  void *jac_work = nullptr;
+  void *eig_work = nullptr;
+  size_t eig_bytes = 0;
+  bool direct = false;     // results go to a caller of tsvd_frpca* / tsvd_merge_svd
+  void *jac_work = nullptr;  // the two-sided eigen-solve's buffers (direct only)
   size_t jac_bytes = 0;
+  double *dv = nullptr, *dt = nullptr, *dh = nullptr;  // [nmax][256*256] its refinement
+  double **dh_ptrs = nullptr;  // device: dh + i 256^2 for each problem i
+  int32_t *eig_stat = nullptr;  // device: most sweeps of an eigen-solve (eig_sweeps_fetch)
   void **dptr = nullptr;   // device pointer-array area
   void **hptr = nullptr;   // pinned staging for the pointer arrays
   size_t ptr_slots = 0;
@@ -31,9 +37,6 @@ struct FrpcaWork {
   CUtensorMap *tmap_host = nullptr;  // pinned staging for them
   size_t tmap_slots = 0;
   int last_sweeps = 0;
-  double *dv = nullptr, *dt = nullptr, *dh = nullptr;  // [nmax][256*256] eigen refinement
-  double **dh_ptrs = nullptr;  // device: dh + i 256^2 for each problem i
-  int last_refine_sweeps = 0;
   // merges wider than 256 columns (allocated on first use)
   float *wm = nullptr;      // [nprob][|S|][n] the concatenated children
   float *wv = nullptr;      // [nprob][n][256] basis of the right singular subspace
@@ -48,8 +51,14 @@ struct FrpcaWork {
   int wide_iters = 0;       // subspace iterations of the last wide merge level
 };
 
-tsvd_status frpca_work_alloc(FrpcaWork &W, int nmax, int64_t rows_max, int sp, int l, int d);
+// Direct eigen-solves of up to this many columns take the one-sided solver:
+// there its results and the two-sided one's agree to 1e-5 (see jacobi.cu).
+constexpr int kDirectOneSided = 48;
+
+tsvd_status frpca_work_alloc(FrpcaWork &W, int nmax, int64_t rows_max, int sp, int l, int d,
+                             bool direct = false);
 void frpca_work_free(FrpcaWork &W);
+tsvd_status eig_sweeps_fetch(FrpcaWork &W, cudaStream_t st);
 
 struct SparseBlock;
 

@@ -182,7 +182,7 @@ tsvd_status frpca_host(int32_t nrows, int32_t ncols, const HostBlock &H, int32_t
     }
     TSVD_CUDA(cudaMemcpyAsync(dcmap.p, H.cmap.data(), sizeof(int32_t) * nc, cudaMemcpyHostToDevice, st));
     FrpcaWork W;
-    s1 = frpca_work_alloc(W, 1, nc, sp, l, k);
+    s1 = frpca_work_alloc(W, 1, nc, sp, l, k, true);
     if (s1 == TSVD_OK) {
       FrpcaProblem P;
       P.block = 0;
@@ -286,7 +286,7 @@ extern "C" void frPCA(mat_csr *A, mat **U, mat **S, mat **V, int k, int q) {
 // truncated_singular_value_decomposition (matrix_vector_functions_intel_mkl.c
 // :1259-1300): US = U_d diag(s_d) of the dense rows x cols matrix M
 // (column-major, as the reference's mat), sigma = s_d descending. The tree
-// merge's own path: compensated Gram, Jacobi refined in fp64, and for more
+// merge's own path: compensated Gram, eigen-solve, and for more
 // than 256 columns the subspace iteration of the wide merge.
 extern "C" tsvd_status tsvd_merge_svd(int32_t rows, int32_t cols, const double *M, int32_t d,
                                       double *US, double *sigma) {
@@ -304,7 +304,7 @@ extern "C" tsvd_status tsvd_merge_svd(int32_t rows, int32_t cols, const double *
   cudaStream_t st;
   TSVD_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   FrpcaWork W;
-  tsvd_status s1 = frpca_work_alloc(W, 1, rows, sp, std::min(kLp, d + 5), d);
+  tsvd_status s1 = frpca_work_alloc(W, 1, rows, sp, std::min(kLp, d + 5), d, true);
   std::vector<float> hu((size_t)rows * d), hs(d);
   if (s1 == TSVD_OK) s1 = merge_matrix(W, m.data(), rows, cols, dout.p, dsig.p, st);
   if (s1 == TSVD_OK) {

@@ -44,6 +44,8 @@ inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
 // Grid size for grid-stride kernels: a multiple of the SM count.
 int grid_for(int64_t work_items, int threads_per_block, int blocks_per_sm = 8);
 int sm_count();
+// Raises (never lowers) a kernel's dynamic shared-memory ceiling.
+tsvd_status raise_smem_ceiling(const void *fn, size_t bytes);
 
 // ---------------------------------------------------------------- scan/sort
 // Exclusive prefix sum of n int32 counts into int64 offsets (out has n+1
@@ -146,17 +148,23 @@ tsvd_status apply_right_batched(const float *const *x, const int32_t *rows,
                                 const float *const *colscale, float *const *y,
                                 int ldy, __half *const *yhi, __half *const *ylo,
                                 float split_scale, int nprob, cudaStream_t st);
-// Two-sided cyclic Jacobi on G[b] (n x n fp64 in, fp32 work): eigenvalues
-// (descending) and eigenvectors V[b] (n x n row-major fp32, column j is the
-// eigenvector of lambda[j]).
-// refine = 1: g[b] = V^T G V for approximate eigenvectors V (nearly
-// diagonal); the diagonal is carried in fp64 (see jacobi_kernel) and the
-// rotations are replayed onto vinit[b] (V, n x n row-major), so v[b] = V R.
+// Eigenpairs of the Grams G[b] (n x n fp64, 2 <= n <= 256) to high relative
+// accuracy: lambda[b] (n values, descending) and the leading nv eigenvectors,
+// column j of V[b] (n x n row-major fp32; the other columns are not written).
+// *sweeps (device) becomes the maximum of itself and the sweeps of any problem.
+tsvd_status eig_gram_batched(double *const *g, int n, int nv, float *const *lambda,
+                             float *const *v, int nprob, void *work, size_t work_bytes,
+                             int32_t *sweeps, cudaStream_t st);
+size_t eig_work_bytes(int n, int nprob);
+// The same by a two-sided cyclic Jacobi on G[b] (n x n fp64 in, fp32 work),
+// all n eigenvectors. refine = 1: g[b] = V^T G V for approximate eigenvectors V
+// (nearly diagonal); the diagonal is carried in fp64 (see jacobi_kernel) and
+// the rotations are replayed onto vinit[b] (V, n x n row-major), so v[b] = V R.
 // v may alias vinit.
 tsvd_status jacobi_eig_batched(double *const *g, int n, float *const *lambda,
                                float *const *v, int nprob, void *work,
                                size_t work_bytes, cudaStream_t st,
-                               int *sweeps_out, int refine = 0,
+                               int32_t *sweeps, int refine = 0,
                                const float *const *vinit = nullptr);
 size_t jacobi_work_bytes(int n, int nprob);
 

@@ -441,9 +441,9 @@ extern "C" tsvd_status tsvd_session_footprint(const tsvd_config *c, int64_t expe
   b += nodes * S * d * 4 + nodes * d * 4 + S * d * 4;                   // tree factors
   const double rows_max = n - (P - 1) * std::floor(n / P) + 1;
   b += P * rows_max * kLp * 8 + P * sp * 256 * 4;                      // X hi/lo, Z
-  b += P * sp * kLp * 8 + P * 65536 * (8 + 4 + 24) + P * 2048 * 4;     // Y, Q, G, V, refine
+  b += P * sp * kLp * 8 + P * 65536 * (8 + 4) + P * 2048 * 4;          // Y, Q, G, V
   b += (std::min(P * std::ceil(std::max(rows_max, sp) / 128), 2048.0) + P) * 65536 * 8;  // Grams
-  b += P * 30.0 * 255 * 128 * 8;                                        // Jacobi rotation logs
+  b += P * (257 * 256 * 8 + 2048);                                        // eigen-solve
   if (c->lp_right_factor) b += n * kLp * 4 + P * S * d * 4 + 8 * n;
   *bytes = (int64_t)(b * 1.05) + (64ll << 20);
   return TSVD_OK;
@@ -832,7 +832,6 @@ static tsvd_status stage_factorize(tsvd_session *s, FactorJob &job, cudaStream_t
       TSVD_TRY(plain_block_build(s->pbw, src, s->nnz_h[b], st));
       probs[i].sparse = &s->pbw.blk;
       TSVD_TRY(frpca_batch(s->fw, &probs[i], 1, s->q, s->cfg.seed, s->S, st, &ssum[i]));
-      job.stats.eig_refine_sweeps = std::max(job.stats.eig_refine_sweeps, s->fw.last_refine_sweeps);
     }
   } else if (s->cfg.block_path == TSVD_BLOCKS_DENSE) {
     TSVD_TRY(frpca_batch(s->fw, probs.data(), nf, s->q, s->cfg.seed, s->S, st, ssum.data()));
@@ -840,7 +839,6 @@ static tsvd_status stage_factorize(tsvd_session *s, FactorJob &job, cudaStream_t
     TSVD_TRY(factorize_two_paths(s, job, probs, ssum, st));
   }
   job.stats.eig_sweeps_frpca = s->fw.last_sweeps;
-  job.stats.eig_refine_sweeps = std::max(job.stats.eig_refine_sweeps, s->fw.last_refine_sweeps);
   // Residual ||A - U S V^T||_F = sqrt(||A||^2 - sum sigma^2) for an orthonormal
   // basis (the reference forms the dense product, Tree_u_NC.cpp:158-204).
   if (job.iter >= s->cfg.lazy_update_start_iter - 1)
@@ -877,9 +875,7 @@ static tsvd_status stage_merge(tsvd_session *s, FactorJob &job, cudaStream_t st)
     } else {
       TSVD_TRY(merge_batch(s->fw, probs.data(), (int)probs.size(), h, s->S, mode, st));
     }
-    job.stats.eig_sweeps_merge = std::max(job.stats.eig_sweeps_merge, s->fw.last_sweeps);
     job.stats.merge_subspace_iters = std::max(job.stats.merge_subspace_iters, s->fw.wide_iters);
-    job.stats.eig_refine_sweeps = std::max(job.stats.eig_refine_sweeps, s->fw.last_refine_sweeps);
     job.stats.merged_nodes += (int)probs.size();
     if (root) {
       TSVD_CUDA(cudaMemcpyAsync(s->node_b(0), s->embedding, sizeof(float) * s->node_elems(),
@@ -895,7 +891,9 @@ static tsvd_status stage_merge(tsvd_session *s, FactorJob &job, cudaStream_t st)
     std::sort(next.begin(), next.end());
     level.swap(next);
   }
+  TSVD_TRY(eig_sweeps_fetch(s->fw, st));
   TSVD_CUDA(cudaStreamSynchronize(st));
+  job.stats.eig_sweeps_merge = s->fw.last_sweeps;
   return TSVD_OK;
 }
 
