@@ -11,6 +11,8 @@ direction and length are off by sqrt(2040) 2^-24 = 2.7e-6; four times that."""
 import numpy as np
 import pytest
 
+from oracle.tree_oracle import frpca as oracle_frpca, gaussian_matrix
+
 pytestmark = pytest.mark.gpu
 TOL = 1.1e-5
 
@@ -54,3 +56,23 @@ def test_blocks_of_low_rank_stay_finite():
             B, sig = s.tree_factor(node)
             assert np.isfinite(B).all() and np.isfinite(sig).all(), node
             assert (np.diff(sig) <= 1e-6 * sig[0]).all(), node
+
+
+@pytest.mark.parametrize("k", [1, 26, 27, 28, 59, 60, 91, 92, 123, 124, 128, 139])
+def test_frpca_basis_at_the_panel_edges(k):
+    """CholeskyQR's factor and inverse (csrc/chol.cu) at basis widths k + 5
+    around its 32-column panels: U = Q V is orthonormal. Two passes leave Q
+    orthonormal to about l 2^-24 = 9e-6, V's columns are up to 4.4e-5 short;
+    their sum, doubled for the squares, is 1.1e-4."""
+    import tsvd_gb300 as T
+    rng = np.random.default_rng(k)
+    m, n = 300, 500
+    q1 = np.linalg.qr(rng.standard_normal((m, m)))[0]
+    q2 = np.linalg.qr(rng.standard_normal((n, m)))[0]
+    A = (q1 * np.geomspace(10, 0.1, m)) @ q2.T
+    U, S, V = T.frpca(np.arange(m + 1) * n, np.tile(np.arange(n), m), A.ravel(), (m, n), k, 6)
+    assert np.abs(U.T @ U - np.eye(k)).max() <= 1.1e-4
+    # frPCA's own values, not the matrix's: a few passes over a slow decay
+    S0 = oracle_frpca(A, k, 6, omega=gaussian_matrix(20231, 0, n, k + 5))[1][::-1]
+    lead = max(1, k // 2)
+    assert np.allclose(S[:lead], S0[:lead], rtol=2e-3)

@@ -11,13 +11,12 @@
 //    5-stage pipeline of full / empty mbarriers.
 //  gram_batched : X^T X with error-free products and compensated sums per
 //    row chunk, chunks summed in fp64 (Code/frpca.c:101, cblas_dgemm TN).
-//  chol_inverse_batched / apply_right_batched : CholeskyQR2 normalization,
-//    replacing LUfraction (Code/frpca.c:4-41); the span of the basis, which
-//    is all the power iteration keeps, is the same.
+//  apply_right_batched : X W, with chol_inverse_batched (chol.cu) the
+//    CholeskyQR2 normalization replacing LUfraction (Code/frpca.c:4-41); the
+//    span of the basis, which is all the power iteration keeps, is the same.
 #include <algorithm>
 #include <map>
 #include <mutex>
-#include <cfloat>
 #include <cstring>
 
 #include "internal.h"
@@ -466,73 +465,6 @@ __global__ void gram_reduce_kernel(const double *__restrict__ work, int nchunks,
   }
 }
 
-// ------------------------------------------------------------------ Cholesky
-constexpr int CHOL_THREADS = 512;
-__global__ void __launch_bounds__(CHOL_THREADS) chol_inverse_kernel(double *const *gs,
-                                                                    float *const *ts, int l) {
-  extern __shared__ __align__(16) float sm[];
-  const int LD = l + 1;
-  float *L = sm;              // [l][LD]
-  float *Li = sm + l * LD;    // [l][LD]
-  __shared__ int drop[kLp];
-  __shared__ float tol;
-  const double *G = gs[blockIdx.x];
-  float *T = ts[blockIdx.x];
-  for (int i = threadIdx.x; i < l * l; i += blockDim.x) {
-    int r = i / l, c = i % l;
-    L[r * LD + c] = (float)G[i];
-    Li[r * LD + c] = 0.f;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float mx = 0.f;
-    for (int i = 0; i < l; ++i) mx = fmaxf(mx, L[i * LD + i]);
-    tol = mx * 1e-12f;
-  }
-  __syncthreads();
-  for (int k = 0; k < l; ++k) {
-    if (threadIdx.x == 0) {
-      float d = L[k * LD + k];
-      if (!(d > tol) || !(d > 0.f)) {
-        drop[k] = 1;
-        L[k * LD + k] = 1.f;
-      } else {
-        drop[k] = 0;
-        L[k * LD + k] = sqrtf(d);
-      }
-    }
-    __syncthreads();
-    const float piv = L[k * LD + k];
-    const int dk = drop[k];
-    for (int i = k + 1 + threadIdx.x; i < l; i += blockDim.x)
-      L[i * LD + k] = dk ? 0.f : L[i * LD + k] / piv;
-    __syncthreads();
-    const int n = l - k - 1;
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-      int i = k + 1 + t / n, j = k + 1 + t % n;
-      if (j <= i) L[i * LD + j] -= L[i * LD + k] * L[j * LD + k];
-    }
-    __syncthreads();
-  }
-  // Li = L^{-1} by forward substitution, one column per thread.
-  for (int j = threadIdx.x; j < l; j += blockDim.x) {
-    Li[j * LD + j] = 1.f / L[j * LD + j];
-    for (int i = j + 1; i < l; ++i) {
-      float s = 0.f;
-      for (int k = j; k < i; ++k) s += L[i * LD + k] * Li[k * LD + j];
-      Li[i * LD + j] = -s / L[i * LD + i];
-    }
-  }
-  __syncthreads();
-  // T = R^{-1} = (L^{-1})^T, dropped directions zeroed.
-  for (int i = threadIdx.x; i < l * kLp; i += blockDim.x) {
-    int r = i / kLp, c = i % kLp;
-    float v = 0.f;
-    if (c < l && r < l && c >= r && !drop[c]) v = Li[c * LD + r];
-    T[i] = v;
-  }
-}
-
 // ------------------------------------------------------------------ X * W
 // Y = X W diag(colscale) (rows x n_out, written up to ldy <= 144 columns,
 // zero past n_out), optionally split into fp16 hi/lo. Register tiles: 256
@@ -820,185 +752,6 @@ tsvd_status gram_batched(const float *const *x, const int32_t *rows, int max_row
   TSVD_LAUNCH_CHECK();
   gram_reduce_kernel<<<dim3((unsigned)ceil_div((int64_t)l * l, 256), nprob), 256, 0, st>>>(
       work, nchunks, l, g, nprob);
-  TSVD_LAUNCH_CHECK();
-  return TSVD_OK;
-}
-
-tsvd_status chol_inverse_batched(double *const *g, float *const *t, int l, int nprob,
-                                 cudaStream_t st) {
-  if (nprob == 0) return TSVD_OK;
-  if (l > kLp) return fail(TSVD_ERR_INVALID, "chol: l=%d > %d", l, kLp);
-  size_t smem = (size_t)2 * l * (l + 1) * sizeof(float);
-  TSVD_TRY(raise_smem_ceiling((const void *)chol_inverse_kernel, smem));
-  chol_inverse_kernel<<<nprob, CHOL_THREADS, smem, st>>>(g, t, l);
-  TSVD_LAUNCH_CHECK();
-  return TSVD_OK;
-}
-
-// One block per problem: the lower Cholesky factor of G in fp64 in global
-// memory (it stays in L2), right-looking, a column per step. Directions whose
-// pivot falls below 1e-13 of the largest diagonal entry are dropped: unit
-// pivot, zero column, flag 1.0 after the factor (work: l*l + l doubles).
-__global__ void __launch_bounds__(1024) chol_wide_kernel(double *const *gs, double *work, int l) {
-  __shared__ double tol;
-  const double *G = gs[blockIdx.x];
-  double *A = work + (int64_t)blockIdx.x * (l * l + l);
-  double *drop = A + (int64_t)l * l;
-  for (int i = threadIdx.x; i < l * l; i += blockDim.x) A[i] = G[i];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double mx = 0.0;
-    for (int i = 0; i < l; ++i) mx = fmax(mx, A[(int64_t)i * l + i]);
-    tol = mx * 1e-13;
-  }
-  __syncthreads();
-  for (int k = 0; k < l; ++k) {
-    if (threadIdx.x == 0) {
-      const double d = A[(int64_t)k * l + k];
-      const bool dk = !(d > tol) || !(d > 0.0);
-      drop[k] = dk ? 1.0 : 0.0;
-      A[(int64_t)k * l + k] = dk ? 1.0 : sqrt(d);
-    }
-    __syncthreads();
-    const double piv = A[(int64_t)k * l + k];
-    const bool dk = drop[k] != 0.0;
-    for (int i = k + 1 + threadIdx.x; i < l; i += blockDim.x)
-      A[(int64_t)i * l + k] = dk ? 0.0 : A[(int64_t)i * l + k] / piv;
-    __syncthreads();
-    const int n = l - k - 1;
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-      const int i = k + 1 + t / n, j = k + 1 + t % n;
-      if (j <= i) A[(int64_t)i * l + j] -= A[(int64_t)i * l + k] * A[(int64_t)j * l + k];
-    }
-    __syncthreads();
-  }
-}
-
-// y = x R^-1 with R = L^T, one thread per row: y_j = (x_j - sum_{k<j} y_k
-// L[j][k]) / L[j][j] in fp64, dropped directions 0. x, y: rows x l (ld l) per
-// problem at stride `stride`.
-__global__ void trsm_rows_kernel(const float *__restrict__ x, float *__restrict__ y,
-                                 const double *__restrict__ work, int rows, int l,
-                                 int64_t stride) {
-  const int prob = blockIdx.y;
-  const double *L = work + (int64_t)prob * (l * l + l);
-  const double *drop = L + (int64_t)l * l;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
-    const float *xr = x + prob * stride + (int64_t)r * l;
-    float *yr = y + prob * stride + (int64_t)r * l;
-    for (int j = 0; j < l; ++j) {
-      double s = xr[j];
-      const double *Lj = L + (int64_t)j * l;
-      for (int k = 0; k < j; ++k) s -= (double)yr[k] * Lj[k];
-      yr[j] = drop[j] != 0.0 ? 0.f : (float)(s / Lj[j]);
-    }
-  }
-}
-
-// Shifted Cholesky in fp32 for the basis of a subspace iteration: K + s I =
-// L L^T with s = shift * trace(K) / l, so no direction is dropped and the
-// result R^{-1} = L^{-T} makes a well-conditioned (not exactly orthonormal)
-// basis. One block per problem, packed lower triangle in shared memory; L
-// goes out packed (row i at i(i+1)/2). K: l x l fp32, problem b at b * l * l.
-__global__ void __launch_bounds__(1024) chol_shift_kernel(const float *__restrict__ K,
-                                                          float *__restrict__ Lout, int l,
-                                                          float shift) {
-  extern __shared__ float Lp[];  // l (l + 1) / 2
-  __shared__ float tr;
-  const float *Kb = K + (int64_t)blockIdx.x * l * l;
-  float *Lb = Lout + (int64_t)blockIdx.x * l * (l + 1) / 2;
-  for (int t = threadIdx.x; t < l * (l + 1) / 2; t += blockDim.x) {
-    int i = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
-    while ((i + 1) * (i + 2) / 2 <= t) ++i;
-    while (i * (i + 1) / 2 > t) --i;
-    const int j = t - i * (i + 1) / 2;
-    Lp[t] = Kb[(int64_t)i * l + j];
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float acc = 0.f;
-    for (int i = 0; i < l; ++i) acc += Lp[i * (i + 1) / 2 + i];
-    tr = fmaxf(acc, FLT_MIN) * shift / (float)l;
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < l; i += blockDim.x) Lp[i * (i + 1) / 2 + i] += tr;
-  __syncthreads();
-  for (int k = 0; k < l; ++k) {
-    const int kk = k * (k + 1) / 2 + k;
-    if (threadIdx.x == 0) Lp[kk] = sqrtf(fmaxf(Lp[kk], tr));
-    __syncthreads();
-    const float piv = Lp[kk];
-    for (int i = k + 1 + threadIdx.x; i < l; i += blockDim.x) Lp[i * (i + 1) / 2 + k] /= piv;
-    __syncthreads();
-    const int n = l - k - 1;
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-      const int i = k + 1 + t / n, j = k + 1 + t % n;
-      if (j <= i) Lp[i * (i + 1) / 2 + j] -= Lp[i * (i + 1) / 2 + k] * Lp[j * (j + 1) / 2 + k];
-    }
-    __syncthreads();
-  }
-  for (int t = threadIdx.x; t < l * (l + 1) / 2; t += blockDim.x) Lb[t] = Lp[t];
-}
-
-// y = x L^{-T}, one warp per row: y_j = (x_j - sum_{k<j} y_k L[j][k]) / L[j][j]
-// with the dot product split over the lanes; L packed in shared memory, the
-// row's y in the warp's shared slice. x, y: rows x l, problem b at b * stride.
-__global__ void __launch_bounds__(1024) trsm_warp_kernel(const float *__restrict__ x,
-                                                         float *__restrict__ y,
-                                                         const float *__restrict__ Lpk, int rows,
-                                                         int l, int64_t stride) {
-  extern __shared__ float sm[];
-  float *Lp = sm;                                   // l (l + 1) / 2
-  float *ys = sm + ((l * (l + 1) / 2 + 3) & ~3);    // [warps][l]
-  const int prob = blockIdx.y;
-  const float *Lb = Lpk + (int64_t)prob * l * (l + 1) / 2;
-  for (int t = threadIdx.x; t < l * (l + 1) / 2; t += blockDim.x) Lp[t] = Lb[t];
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  float *yw = ys + warp * l;
-  for (int r = blockIdx.x * nwarps + warp; r < rows; r += gridDim.x * nwarps) {
-    const float *xr = x + prob * stride + (int64_t)r * l;
-    float *yr = y + prob * stride + (int64_t)r * l;
-    for (int j = 0; j < l; ++j) {
-      const float *Lj = Lp + j * (j + 1) / 2;
-      float part = 0.f;
-      for (int k = lane; k < j; k += 32) part = fmaf(yw[k], Lj[k], part);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(kFull, part, o);
-      const float v = (xr[j] - part) / Lj[j];
-      if (lane == 0) yw[j] = v;
-      __syncwarp();
-    }
-    for (int j = lane; j < l; j += 32) yr[j] = yw[j];
-    __syncwarp();
-  }
-}
-
-tsvd_status chol_shift_solve_batched(const float *K, float *Lpk, const float *x, float *y,
-                                     int rows, int l, int64_t stride, float shift, int nprob,
-                                     cudaStream_t st) {
-  if (nprob == 0) return TSVD_OK;
-  if (l > 256 || l < 1) return fail(TSVD_ERR_INVALID, "chol shift: l=%d", l);
-  const size_t csm = (size_t)l * (l + 1) / 2 * sizeof(float);
-  const size_t tsm = (((size_t)l * (l + 1) / 2 + 3) & ~(size_t)3) * sizeof(float) +
-                     (size_t)32 * l * sizeof(float);
-  if (csm > 48 * 1024) TSVD_TRY(raise_smem_ceiling((const void *)chol_shift_kernel, csm));
-  if (tsm > 48 * 1024) TSVD_TRY(raise_smem_ceiling((const void *)trsm_warp_kernel, tsm));
-  chol_shift_kernel<<<nprob, 1024, csm, st>>>(K, Lpk, l, shift);
-  TSVD_LAUNCH_CHECK();
-  const int blocks = (int)std::min<int64_t>(ceil_div(rows, 32), 2 * sm_count() / std::max(nprob, 1) + 1);
-  trsm_warp_kernel<<<dim3(blocks, nprob), 1024, tsm, st>>>(x, y, Lpk, rows, l, stride);
-  TSVD_LAUNCH_CHECK();
-  return TSVD_OK;
-}
-
-tsvd_status chol_solve_wide_batched(double *const *g, double *work, const float *x, float *y,
-                                    int rows, int l, int64_t stride, int nprob, cudaStream_t st) {
-  if (nprob == 0) return TSVD_OK;
-  if (l > 256 || l < 1) return fail(TSVD_ERR_INVALID, "chol wide: l=%d", l);
-  chol_wide_kernel<<<nprob, 1024, 0, st>>>(g, work, l);
-  TSVD_LAUNCH_CHECK();
-  trsm_rows_kernel<<<dim3(ceil_div(rows, 128), nprob), 128, 0, st>>>(x, y, work, rows, l, stride);
   TSVD_LAUNCH_CHECK();
   return TSVD_OK;
 }

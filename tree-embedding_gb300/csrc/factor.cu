@@ -240,7 +240,7 @@ void frpca_work_free(FrpcaWork &W) {
   cudaFreeHost(W.hptr); cudaFree(W.dint); cudaFreeHost(W.hint);
   cudaFree(W.tmap_dev); cudaFreeHost(W.tmap_host);
   cudaFree(W.wm); cudaFree(W.wv); cudaFree(W.ww); cudaFree(W.wy); cudaFree(W.wy2);
-  cudaFree(W.wchol); cudaFree(W.wnorm); cudaFree(W.wk);
+  cudaFree(W.wnorm); cudaFree(W.wk);
   cudaFree(W.jac_work); cudaFree(W.dv); cudaFree(W.dt); cudaFree(W.dh); cudaFree(W.dh_ptrs);
   cudaGetLastError();  // the launch checks read this slot: leave nothing from teardown in it
   W = FrpcaWork();
@@ -567,7 +567,7 @@ __global__ void diag_sum_kernel(double *const *g, int l, double *out) {
 }
 
 
-constexpr int64_t kWideK = 256 * 256 + 256 * 257 / 2;  // fp32 Gram + packed factor
+constexpr int64_t kWideK = 256 * 256 + 256 * 288;  // fp32 Gram + chol_factor_floats(256)
 
 // Buffers for up to `nprob` problems of n columns and W.sp rows.
 tsvd_status wide_reserve(FrpcaWork &W, int nprob, int n) {
@@ -575,16 +575,14 @@ tsvd_status wide_reserve(FrpcaWork &W, int nprob, int n) {
   const size_t need = (size_t)nprob * nsrc * n;
   if (need <= W.wide_cap && nprob <= W.wide_nprob && n <= W.wide_n && W.wm) return TSVD_OK;
   cudaFree(W.wm); cudaFree(W.wv); cudaFree(W.ww); cudaFree(W.wy); cudaFree(W.wy2);
-  cudaFree(W.wchol); cudaFree(W.wnorm); cudaFree(W.wk);
+  cudaFree(W.wnorm); cudaFree(W.wk);
   W.wm = W.wv = W.ww = W.wy = W.wy2 = W.wnorm = W.wk = nullptr;
-  W.wchol = nullptr;
   W.wide_cap = 0;
   TSVD_CUDA(cudaMalloc(&W.wm, need * sizeof(float)));
   TSVD_CUDA(cudaMalloc(&W.wv, (size_t)nprob * n * 256 * sizeof(float)));
   TSVD_CUDA(cudaMalloc(&W.ww, (size_t)nprob * n * 256 * sizeof(float)));
   TSVD_CUDA(cudaMalloc(&W.wy, (size_t)nprob * nsrc * 256 * sizeof(float)));
   TSVD_CUDA(cudaMalloc(&W.wy2, (size_t)nprob * nsrc * 256 * sizeof(float)));
-  TSVD_CUDA(cudaMalloc(&W.wchol, (size_t)nprob * 2 * 256 * 256 * sizeof(double)));
   TSVD_CUDA(cudaMalloc(&W.wnorm, (size_t)nprob * n * sizeof(float)));
   TSVD_CUDA(cudaMalloc(&W.wk, (size_t)nprob * kWideK * sizeof(float)));
   W.wide_cap = need;
@@ -617,7 +615,7 @@ tsvd_status orthonormalize(FrpcaWork &W, float *x, int64_t xstride, float *y, in
     TSVD_LAUNCH_CHECK();
     TSVD_CUDA(cudaMemcpyAsync(energy, W.sums, sizeof(double) * nprob, cudaMemcpyDeviceToHost, st));
   }
-  TSVD_TRY(chol_solve_wide_batched(d_g, W.wchol, x, y, rows, p, xstride, nprob, st));
+  TSVD_TRY(orth_gram_batched(d_g, p, x, y, rows, xstride, nprob, W.eig_work, W.eig_bytes, st));
   TSVD_CUDA(cudaStreamSynchronize(st));
   return TSVD_OK;
 }
@@ -694,7 +692,7 @@ tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, 
   }
   std::vector<double> energy(nprob), prev(nprob, 0.0);
   // x (rows x p, row-major, problem stride xs) -> y: fp32 Gram (problem i at
-  // W.wk + i p p), shifted fp32 Cholesky (packed factors after all the
+  // W.wk + i p p), shifted fp32 Cholesky (factors after all the
   // Grams), triangular solve.
   const int64_t kp = (int64_t)p * p;
   auto cheap_basis = [&](const float *x, int64_t xs, float *y, int rows) -> tsvd_status {

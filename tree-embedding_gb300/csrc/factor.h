@@ -43,8 +43,7 @@ struct FrpcaWork {
   float *ww = nullptr;      // [nprob][n][256] M^T Y before normalization
   float *wy = nullptr;      // [nprob][|S|][256] M V, then its orthonormal basis
   float *wy2 = nullptr;
-  double *wchol = nullptr;  // [nprob][2][256][256] Cholesky factors
-  float *wk = nullptr;      // [nprob][256*256 + 256*257/2] fp32 Gram + packed factor
+  float *wk = nullptr;      // [nprob][256*256 + 256*288] fp32 Gram + factor
   float *wnorm = nullptr;   // [nprob][n] column norms of M
   size_t wide_cap = 0;      // problems x n x |S| the buffers hold
   int wide_nprob = 0, wide_n = 0;

@@ -127,19 +127,21 @@ size_t gram_work_bytes(int max_rows, int l, int nprob);
 // CholeskyQR step: T[b] = R^{-1} from G[b] (upper triangular, l x kLp fp32).
 tsvd_status chol_inverse_batched(double *const *g, float *const *t, int l,
                                  int nprob, cudaStream_t st);
-// CholeskyQR step for l <= 256: factor G[b] = L L^T in fp64 (work: nprob x
-// (l*l + l) doubles), then y_b = x_b L^{-T} row by row (x, y: rows x l fp32,
-// ld l, problem b at offset b * stride). Directions whose pivot falls below
-// 1e-13 of the largest diagonal entry give zero columns.
-tsvd_status chol_solve_wide_batched(double *const *g, double *work, const float *x, float *y,
-                                    int rows, int l, int64_t stride, int nprob, cudaStream_t st);
 // Cheap step of a subspace iteration (l <= 256): K[b] (l x l fp32, at b l l)
-// + shift * trace/l * I = L L^T in fp32, Lpk (packed, nprob x l(l+1)/2) gets
-// L, y_b = x_b L^{-T}. Keeps every direction; the basis is well-conditioned,
-// not exactly orthonormal.
-tsvd_status chol_shift_solve_batched(const float *K, float *Lpk, const float *x, float *y,
+// + shift * trace/l * I = L L^T in fp32, factor (nprob x chol_factor_floats(l))
+// gets L, y_b = x_b L^{-T} (x, y: rows x l fp32, ld l, problem b at offset
+// b * stride). Keeps every direction; the basis is well-conditioned, not
+// exactly orthonormal.
+size_t chol_factor_floats(int l);
+tsvd_status chol_shift_solve_batched(const float *K, float *factor, const float *x, float *y,
                                      int rows, int l, int64_t stride, float shift, int nprob,
                                      cudaStream_t st);
+// An orthonormal basis of x_b's columns (rows x n fp32, ld n, n <= 256, problem
+// b at offset b * stride) from their Gram G[b] (n x n fp64), in the order of
+// the column norms; dependent columns give zero columns.
+tsvd_status orth_gram_batched(double *const *g, int n, const float *x, float *y, int rows,
+                              int64_t stride, int nprob, void *work, size_t work_bytes,
+                              cudaStream_t st);
 // Y[b] = X[b] * W[b] * diag(colscale[b]); writes fp32 (columns [n_out, ldy)
 // zeroed) and, when yhi/ylo are given, the fp16 split of Y * split_scale.
 tsvd_status apply_right_batched(const float *const *x, const int32_t *rows,
