@@ -21,6 +21,8 @@
 // the same invariant the FIFO leaves behind.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <new>
 
 #include "internal.h"
 #include "ppr.h"
@@ -29,8 +31,23 @@ namespace tsvd {
 
 namespace {
 
-constexpr int kHeavy = 1024;  // neighbours per warp work unit for hub vertices
 constexpr unsigned kFull = 0xffffffffu;
+
+// Neighbours a warp takes in one piece; vertices with more are split into
+// units for push_heavy_kernel. In a large round long pieces cost nothing (other
+// warps have other items), and each unit is a slot and a weight read more. In
+// a small one a piece is what the round waits for: 1024 neighbours take one
+// warp 30 us, 128 take 5 (the tail of a push is some 50 such rounds). Rounds of
+// up to 2^18 items cannot overflow the slots.
+__device__ __forceinline__ int32_t piece_for(int32_t nitems) {
+  return nitems < (1 << 18) ? 128 : 1024;
+}
+
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
 
 // Sets the bit of (u, chunk c) in a chunk-major bitset (bit c * n + u). The
 // result is unused, so this is a fire-and-forget reduction (RED.OR). The
@@ -79,27 +96,44 @@ __device__ __forceinline__ void scatter_range(const PushArgs &a, const int32_t *
   for (int32_t jb = j0; jb < j1; jb += 32) {
     const int32_t jn = min(32, j1 - jb);
     const int32_t next = lane < j1 - jb - 32 ? __ldg(nb + jb + 32 + lane) : 0;
+    // the touched bit of the neighbour this lane loaded, as it is now in L2
+    const int64_t idx = (int64_t)c * a.n + mine;
+    const uint32_t bit = 1u << (idx & 31);
+    const uint32_t seen = lane < jn ? __ldcg(a.tflag + (idx >> 5)) : bit;
     for (int32_t t = 0; t < jn; t += 2) {
       const int32_t u = __shfl_sync(kFull, mine, (t + half) & 31);
       if (act && t + half < jn) atomicAdd(rc + (int64_t)u * (kChunk / 4), w4);
     }
-    // each lane marks the neighbour it loaded: 32 independent reductions
-    if (lane < jn) mark_pair(a.tflag, mine, c, a.n);
+    // Each lane marks the neighbour it loaded, unless it is marked: a reduction
+    // costs L2 a sector like each of the run's, of which the scatter is bound,
+    // and in a dense round 28 of 29 marks change nothing.
+    if (!(seen & bit)) atomicOr(a.tflag + (idx >> 5), bit);
     mine = next;
   }
 }
 
-__global__ void __launch_bounds__(256) push_kernel(PushArgs a) {
+// One warp per item, a fixed share of the items each, on a grid of resident
+// blocks (5 a SM; the blocks of a second wave, as with 8 a SM, ran alone at the
+// end). What bounds a dense round is L2's rate of reducing 32-byte sectors:
+// 200-238 G/s here, and 205 G/s for whole random runs that all hit L2 (25.6 G
+// runs/s; half runs 52 G/s). Sharing the items out through a counter kept every
+// SM busy and was slower, its atomics queueing behind the reductions.
+__global__ void __launch_bounds__(256, 5) push_kernel(PushArgs a) {
   const int lane = threadIdx.x & 31;
-  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int32_t nitems = *a.front_count;
+  const int32_t gw = (int32_t)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+  const int32_t nw = (int32_t)(((int64_t)gridDim.x * blockDim.x) >> 5);
+  const int32_t nlight = a.front_count[0], nitems = nlight + a.front_count[kHighCount];
+  const int32_t piece = piece_for(nitems);
+  auto item = [&](int32_t i) {
+    return __ldg(i < nlight ? a.front + i : a.front + (a.cap - 1 - (i - nlight)));
+  };
+  if (gw == 0 && lane == 0) a.stats[kStatSlots * 4] = global_ns();
   StatAcc acc;
-  int2 it = gw < nitems ? __ldg(a.front + gw) : make_int2(0, 0);
-  for (int64_t i = gw; i < nitems; i += nw) {
+  int2 it = gw < nitems ? item(gw) : make_int2(0, 0);
+  for (int32_t i = gw; i < nitems; i += nw) {
     const int32_t v = it.x, c = it.y;
     // the warp's next item is loaded while this one is pushed
-    it = i + nw < nitems ? __ldg(a.front + i + nw) : make_int2(0, 0);
+    it = i + nw < nitems ? item(i + nw) : make_int2(0, 0);
     // Everything the item needs that does not depend on its residues is
     // requested at once: degree, row start, reserve line, first neighbour ids
     // (only this warp writes the reserve of (v, chunk c) in a round).
@@ -158,10 +192,10 @@ __global__ void __launch_bounds__(256) push_kernel(PushArgs a) {
       acc.items += 1;
       acc.iedges += (unsigned long long)d;
     }
-    if (d > kHeavy) {
+    if (d > piece) {
       // Hub vertex: park the lane weights and split the neighbour list into
-      // kHeavy-sized units processed by push_heavy_kernel.
-      const int32_t units = (d + kHeavy - 1) / kHeavy;
+      // piece-sized units processed by push_heavy_kernel.
+      const int32_t units = (d + piece - 1) / piece;
       int32_t slot = 0, u0 = 0, ok = 0;
       if (lane == 0) {
         slot = atomicAdd(a.heavy_count, 1);
@@ -178,7 +212,7 @@ __global__ void __launch_bounds__(256) push_kernel(PushArgs a) {
       }
       if (units_reserved)
         for (int32_t k = lane; k < units; k += 32)
-          a.units[u0 + k] = make_int2(ok ? slot : -1, k * kHeavy);
+          a.units[u0 + k] = make_int2(ok ? slot : -1, k * piece);
       if (ok) continue;
       // buffers full: process this hub inline
     }
@@ -189,17 +223,18 @@ __global__ void __launch_bounds__(256) push_kernel(PushArgs a) {
 
 __global__ void __launch_bounds__(256) push_heavy_kernel(PushArgs a) {
   const int lane = threadIdx.x & 31;
-  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int32_t gw = (int32_t)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+  const int32_t nw = (int32_t)(((int64_t)gridDim.x * blockDim.x) >> 5);
   const int32_t nunits = min(*a.unit_count, a.unit_cap);
-  for (int64_t i = gw; i < nunits; i += nw) {
-    int2 u = a.units[i];
+  const int32_t piece = piece_for(a.front_count[0] + a.front_count[kHighCount]);
+  for (int32_t i = gw; i < nunits; i += nw) {
+    const int2 u = a.units[i];
     if (u.x < 0) continue;
-    int2 it = a.heavy_item[u.x];
+    const int2 it = a.heavy_item[u.x];
     const float2 w = reinterpret_cast<const float2 *>(a.heavy_w)[(int64_t)u.x * 32 + lane];
     const int32_t d = a.deg[it.x];
     const int32_t *nb = a.nbr + a.off[it.x];
-    const int32_t j1 = min(d, u.y + kHeavy);
+    const int32_t j1 = min(d, u.y + piece);
     const int32_t mine0 = lane < j1 - u.y ? __ldg(nb + u.y + lane) : 0;
     scatter_range(a, nb, it.y, w, u.y, j1, mine0);
   }
@@ -207,79 +242,117 @@ __global__ void __launch_bounds__(256) push_heavy_kernel(PushArgs a) {
 
 // Scan the touched bitset; for each touched (u, chunk) with some residue
 // above theta and deg(u) > 0, append it to the next frontier. Clears the bits.
-// A warp takes the set bits of a word eight at a time: lane group g (4 lanes)
-// reads pair g's 256-byte residue run as sixteen float4 (four per lane), so
-// eight runs are in flight per warp. Padding sources (s >= |S|) hold zero
-// residue.
+// A warp lists the set bits of its words (up to eight) in shared memory and
+// takes them eight at a time: lane group g (4 lanes) reads pair g's 256-byte
+// residue run as sixteen float4 (four per lane), so eight runs are in flight
+// per warp. Padding sources (s >= |S|) hold zero residue. A dense bitset is
+// read at the bandwidth of L2; a sparse one waits for latencies, about two per
+// eight pairs, which is why the pairs of all eight words are taken together
+// (word by word, two bits a word cost as much as eight).
 __global__ void __launch_bounds__(256) collect_kernel(CollectArgs a) {
-  __shared__ int2 buf[2048];
-  __shared__ int32_t nbuf, gbase;
+  __shared__ int2 buf[2048];  // light items from the start, the others from the end
+  __shared__ uint8_t list[8][256];  // bit within the warp's words
+  __shared__ int32_t nbuf[2], gbase[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = lane >> 2, gl = lane & 3;
-  const int64_t words_per_iter = 64;  // 8 warps x 8 words
+  const unsigned below = (1u << lane) - 1u;
+  const int64_t words_per_iter = 8 * a.words;
+  if (a.spent && blockIdx.x == 0 && threadIdx.x < 8) {
+    // the round's counters start at zero again (its scatter kernels are done)
+    if (threadIdx.x == 0) {
+      a.spent[0] = a.spent[kHighCount] = 0;
+      a.clock[1] += global_ns() - a.clock[0];
+    }
+    if (threadIdx.x == 2 || threadIdx.x == 3) a.round[threadIdx.x - 2] = 0;
+  }
   for (int64_t w0 = (int64_t)blockIdx.x * words_per_iter; w0 < a.nwords;
        w0 += (int64_t)gridDim.x * words_per_iter) {
-    if (threadIdx.x == 0) nbuf = 0;
-    // the warp's eight words in one load (lanes 0-7): in the late rounds of a
-    // push almost every word is zero, and eight dependent loads per warp made
-    // the scan of the bitset cost 0.14 ms a round
-    const int64_t wbase = w0 + warp * 8;
-    const uint32_t wv = (lane < 8 && wbase + lane < a.nwords) ? __ldcg(a.tflag + wbase + lane) : 0u;
+    if (threadIdx.x < 2) nbuf[threadIdx.x] = 0;
+    // The warp's words in one load: in the late rounds of a push almost every
+    // word is zero. A small bitset is spread over the warps there are, down to
+    // a word each: with eight words a warp the 125 words of a 4000-vertex graph
+    // kept two blocks busy for 37 us.
+    const int64_t wbase = w0 + warp * a.words;
+    const int wk = lane >> 2;  // this lane's word and byte
+    const bool mine = wk < a.words && wbase + wk < a.nwords;
+    const uint32_t word = mine ? __ldcg(a.tflag + wbase + wk) : 0u;
+    if (word && gl == 0) a.tflag[wbase + wk] = 0;
+    uint32_t byte = (word >> (8 * gl)) & 0xffu;
+    int at = __popc(byte);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(kFull, at, o);
+      if (lane >= o) at += y;
+    }
+    const int total = __shfl_sync(kFull, at, 31);
+    at -= __popc(byte);
+    while (byte) {
+      list[warp][at++] = (uint8_t)(lane * 8 + __ffs(byte) - 1);
+      byte &= byte - 1;
+    }
     __syncthreads();
-    for (int k = 0; k < 8; ++k) {
-      const int64_t wi = wbase + k;
-      if (wi >= a.nwords) break;
-      uint32_t bits = __shfl_sync(kFull, wv, k);
-      if (!bits) continue;
-      if (lane == 0) a.tflag[wi] = 0;
-      while (bits) {
-        // the next (up to) eight set bits, one per lane group
-        uint32_t rest = bits;
-        int mybit = -1;
-        for (int g = 0; g < 8 && rest; ++g) {
-          const int bpos = __ffs(rest) - 1;
-          rest &= rest - 1;
-          if (g == grp) mybit = bpos;
-        }
-        bits = rest;
-        int32_t u = 0, c = 0, du = 0;
-        bool live = mybit >= 0;
-        if (live) {
-          const int64_t idx = wi * 32 + mybit;
-          u = (int32_t)(idx % a.n);
-          c = (int32_t)(idx / a.n);
-          du = a.deg[u];
-          live = du != 0;
-        }
-        const float th = (a.hub_deg > 0 && du < a.hub_deg) ? a.rmax_f : a.theta_f;
-        float m = 0.f;
-        if (live) {
+    const int32_t c0 = (int32_t)(wbase * 32 / a.n), u0 = (int32_t)(wbase * 32 - (int64_t)c0 * a.n);
+    for (int base = 0; base < total; base += 16) {
+      int32_t u[2], c[2], du[2];
+      float4 x[2][4];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {  // two sets of eight pairs in flight
+        const int i = base + 8 * k + grp;
+        u[k] = c[k] = du[k] = 0;
+        if (i < total) {
+          u[k] = u0 + list[warp][i];
+          c[k] = c0;
+          while (u[k] >= a.n) {
+            u[k] -= a.n;
+            ++c[k];
+          }
+          du[k] = __ldg(a.deg + u[k]);
           const float4 *line =
-              reinterpret_cast<const float4 *>(a.r + ppr_cell(u, c * kChunk, a.n));
-          const float4 x0 = __ldcg(line + gl), x1 = __ldcg(line + gl + 4);
-          const float4 x2 = __ldcg(line + gl + 8), x3 = __ldcg(line + gl + 12);
-          const float m0 = fmaxf(fmaxf(fmaxf(x0.x, x0.y), fmaxf(x0.z, x0.w)),
-                                 fmaxf(fmaxf(x1.x, x1.y), fmaxf(x1.z, x1.w)));
-          const float m1 = fmaxf(fmaxf(fmaxf(x2.x, x2.y), fmaxf(x2.z, x2.w)),
-                                 fmaxf(fmaxf(x3.x, x3.y), fmaxf(x3.z, x3.w)));
-          m = fmaxf(m0, m1);
+              reinterpret_cast<const float4 *>(a.r + ppr_cell(u[k], c[k] * kChunk, a.n));
+#pragma unroll
+          for (int q = 0; q < 4; ++q) x[k][q] = __ldcg(line + gl + 4 * q);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) x[k][q] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        float m = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          m = fmaxf(m, fmaxf(fmaxf(x[k][q].x, x[k][q].y), fmaxf(x[k][q].z, x[k][q].w)));
+        const bool live = du[k] != 0;
+        const float th = (a.hub_deg > 0 && du[k] < a.hub_deg) ? a.rmax_f : a.theta_f;
         const unsigned above = __ballot_sync(kFull, live && m > th);
         const unsigned parked =
             __ballot_sync(kFull, live && th > a.rmax_f && m > a.rmax_f) & ~above;
         const unsigned gmask = 0xFu << (grp * 4);
-        if (gl == 0 && live) {
-          if (above & gmask) buf[atomicAdd(&nbuf, 1)] = make_int2(u, c);
-          else if (parked & gmask) mark_pair(a.pend, u, c, a.n);  // for a lower level
+        const bool lead = gl == 0 && live, take = lead && (above & gmask);
+        const bool high = du[k] > a.light;
+        // one shared atomic per class
+        const unsigned mlow = __ballot_sync(kFull, take && !high),
+                       mhigh = __ballot_sync(kFull, take && high);
+        if (mlow | mhigh) {
+          int slot = 0;
+          if (lane < 2) slot = atomicAdd(&nbuf[lane], __popc(lane ? mhigh : mlow));
+          const int low_at = __shfl_sync(kFull, slot, 0), high_at = __shfl_sync(kFull, slot, 1);
+          if (take)
+            buf[high ? 2047 - (high_at + __popc(mhigh & below)) : low_at + __popc(mlow & below)] =
+                make_int2(u[k], c[k]);
         }
+        if (lead && !take && (parked & gmask)) mark_pair(a.pend, u[k], c[k], a.n);  // a lower level
       }
     }
     __syncthreads();
-    if (threadIdx.x == 0) gbase = nbuf ? atomicAdd(a.next_count, nbuf) : 0;
+    if (threadIdx.x < 2)
+      gbase[threadIdx.x] = nbuf[threadIdx.x] ? atomicAdd(a.next_count + kHighCount * threadIdx.x,
+                                                         nbuf[threadIdx.x]) : 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < nbuf; i += blockDim.x) {
-      const int64_t dst = (int64_t)gbase + i;
-      if (dst < a.cap) a.next[dst] = buf[i];
+    for (int i = threadIdx.x; i < nbuf[0] + nbuf[1]; i += blockDim.x) {
+      const int high = i >= nbuf[0], k = high ? i - nbuf[0] : i;
+      const int64_t dst = (int64_t)gbase[high] + k;
+      if (dst < a.cap) a.next[high ? a.cap - 1 - dst : dst] = buf[high ? 2047 - k : k];
       else atomicExch(a.overflow, 1);
     }
     __syncthreads();
@@ -382,7 +455,10 @@ __global__ void init_sources_kernel(const int32_t *__restrict__ sources, int32_t
     r[ppr_cell(v, k, n)] = 1.0f;
     front[k] = make_int2(v, k / kChunk);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *count = nsrc;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    count[0] = nsrc;
+    count[kHighCount] = 0;
+  }
 }
 
 // Zero fill with 16-byte stores (also for p in mapped host memory).
@@ -407,6 +483,27 @@ float largest_float_not_above(double x) {
 }
 
 }  // namespace
+
+// Blocks of 256 threads the kernel keeps resident on the whole GPU.
+static int resident_blocks(const void *fn) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0) != cudaSuccess) {
+    cudaGetLastError();
+    per_sm = 4;
+  }
+  return sm_count() * std::max(per_sm, 1);
+}
+
+static int32_t light_degree(const PprState &P) {
+  return P.cap < kLightPairs ? INT32_MAX : kLightDegree;
+}
+
+// collect_kernel's grid and words per warp for a bitset of nwords words.
+static int collect_grid(int64_t nwords, int *words) {
+  static const int resident = resident_blocks((const void *)collect_kernel);
+  *words = (int)std::max<int64_t>(1, std::min<int64_t>(8, ceil_div(nwords, (int64_t)resident * 8)));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(nwords, 8ll * *words), resident));
+}
 
 tsvd_status ppr_alloc(PprState &P, int32_t n, int32_t nsrc, int32_t sp, bool host_reserve) {
   P.n = n;
@@ -447,13 +544,15 @@ tsvd_status ppr_alloc(PprState &P, int32_t n, int32_t nsrc, int32_t sp, bool hos
   TSVD_CUDA(cudaMalloc(&P.heavy_item, (size_t)P.heavy_cap * sizeof(int2)));
   TSVD_CUDA(cudaMalloc(&P.units, (size_t)P.unit_cap * sizeof(int2)));
   TSVD_CUDA(cudaMalloc(&P.upd, (size_t)n * sizeof(int32_t)));
-  TSVD_CUDA(cudaMalloc(&P.counters, 16 * sizeof(int32_t)));
-  TSVD_CUDA(cudaMemset(P.counters, 0, 16 * sizeof(int32_t)));
-  TSVD_CUDA(cudaMalloc(&P.stats, kStatSlots * 4 * sizeof(unsigned long long)));
-  TSVD_CUDA(cudaMallocHost(&P.host_counters, 16 * sizeof(int32_t)));
+  TSVD_CUDA(cudaMalloc(&P.counters, kCounters * sizeof(int32_t)));
+  TSVD_CUDA(cudaMemset(P.counters, 0, kCounters * sizeof(int32_t)));
+  TSVD_CUDA(cudaMalloc(&P.stats, (kStatSlots * 4 + 2) * sizeof(unsigned long long)));
+  TSVD_CUDA(cudaMallocHost(&P.host_counters, 2 * kCounters * sizeof(int32_t)));
   for (auto &e : P.kev) TSVD_CUDA(cudaEventCreate(&e));
   return TSVD_OK;
 }
+
+static void graph_free(RoundGraph *g);
 
 void ppr_free(PprState &P) {
   cudaFree(P.r);
@@ -468,11 +567,13 @@ void ppr_free(PprState &P) {
   cudaFreeHost(P.host_counters);
   for (auto &e : P.kev)
     if (e) cudaEventDestroy(e);
+  graph_free(P.graph);
   P = PprState();
 }
 
 // counters: [0],[1] frontier counts, [2] heavy count, [3] unit count,
-// [4] overflow flag, [5] number of updated vertices.
+// [4] overflow flag, [5] number of updated vertices, [8],[9] frontier counts of
+// the items that are not light.
 tsvd_status ppr_refresh(PprState &P, const Adjacency &A, const int32_t *sources_dev,
                         bool from_scratch, const PprParams &prm, uint8_t *vmark,
                         cudaStream_t st) {
@@ -482,7 +583,6 @@ tsvd_status ppr_refresh(PprState &P, const Adjacency &A, const int32_t *sources_
     TSVD_TRY(zero_floats(P.p, (size_t)P.n * P.sp, st));
     TSVD_CUDA(cudaMemsetAsync(P.tflag, 0, P.nwords * sizeof(uint32_t), st));
     TSVD_CUDA(cudaMemsetAsync(P.pend, 0, P.nwords * sizeof(uint32_t), st));
-    P.cur = 0;
     init_sources_kernel<<<grid_for(P.nsrc, 256), 256, 0, st>>>(sources_dev, P.nsrc, P.r, P.n,
                                                                   P.front[0], P.counters + 0);
     TSVD_LAUNCH_CHECK();
@@ -500,15 +600,17 @@ tsvd_status ppr_refresh(PprState &P, const Adjacency &A, const int32_t *sources_
   refresh_kernel<<<grid_for((A.n + 31) / 32 * (int64_t)P.chunks * 32, 256, 16), 256, 0, st>>>(ra);
   TSVD_LAUNCH_CHECK();
   // seed the frontier from the touched (vertex, chunk) pairs
-  P.cur = 0;
-  TSVD_CUDA(cudaMemsetAsync(P.counters + 0, 0, sizeof(int32_t), st));
+  TSVD_CUDA(cudaMemsetAsync(P.counters, 0, kCounters * sizeof(int32_t), st));
   CollectArgs ca;
   ca.tflag = P.tflag; ca.nwords = P.nwords; ca.n = P.n; ca.chunks = P.chunks; ca.nsrc = P.nsrc;
   ca.sp = P.sp; ca.r = P.r; ca.deg = A.deg; ca.rmax_f = largest_float_not_above(prm.rmax);
   ca.theta_f = ca.rmax_f; ca.hub_deg = 0; ca.pend = P.pend;
   ca.next = P.front[0]; ca.next_count = P.counters + 0; ca.cap = P.cap;
   ca.overflow = P.counters + 4;
-  collect_kernel<<<grid_for(ceil_div(P.nwords, 64) * 256, 256, 8), 256, 0, st>>>(ca);
+  ca.spent = nullptr;
+  ca.light = light_degree(P);
+  const int gcol = collect_grid(P.nwords, &ca.words);
+  collect_kernel<<<gcol, 256, 0, st>>>(ca);
   TSVD_LAUNCH_CHECK();
   P.seeded = true;
   return TSVD_OK;
@@ -516,17 +618,16 @@ tsvd_status ppr_refresh(PprState &P, const Adjacency &A, const int32_t *sources_
 
 namespace {
 
-// One push (one PPR state), advanced check_every rounds at a time.
+// One push (one PPR state), advanced kRounds rounds at a time.
 struct PushJob {
   PprState *P = nullptr;
   cudaStream_t st = nullptr;
-  PushArgs pa{};
-  CollectArgs ca{};
-  int gpush = 0, gcol = 0;
+  PushArgs pa;  // zeroed by job_begin, padding too: compared as bytes
+  CollectArgs ca;
+  int gpush = 0, gheavy = 0, gcol = 0;
   int level = 0;
   bool done = false;
   int64_t rounds = 0;
-  double kernel_ms = 0;
 };
 
 tsvd_status job_begin(PushJob &J, PprState &P, const Adjacency &A, const PprParams &prm,
@@ -534,8 +635,13 @@ tsvd_status job_begin(PushJob &J, PprState &P, const Adjacency &A, const PprPara
   if (!P.seeded) return fail(TSVD_ERR_STATE, "push before refresh");
   J.P = &P;
   J.st = st;
-  TSVD_CUDA(cudaMemsetAsync(P.stats, 0, kStatSlots * 4 * sizeof(unsigned long long), st));
-  TSVD_CUDA(cudaMemsetAsync(P.counters + 4, 0, sizeof(int32_t), st));
+  TSVD_CUDA(cudaMemsetAsync(P.stats, 0, (kStatSlots * 4 + 2) * sizeof(unsigned long long), st));
+  // every counter but the frontier's (the refresh leaves it in counters[0] and
+  // counters[kHighCount])
+  TSVD_CUDA(cudaMemsetAsync(P.counters + 1, 0, 7 * sizeof(int32_t), st));
+  TSVD_CUDA(cudaMemsetAsync(P.counters + 9, 0, sizeof(int32_t), st));
+  std::memset(&J.pa, 0, sizeof J.pa);
+  std::memset(&J.ca, 0, sizeof J.ca);
   const float rmax_f = largest_float_not_above(prm.rmax);
   PushArgs &pa = J.pa;
   pa.r = P.r; pa.p = P.p; pa.off = A.off; pa.deg = A.deg; pa.nbr = A.nbr;
@@ -544,6 +650,7 @@ tsvd_status job_begin(PushJob &J, PprState &P, const Adjacency &A, const PprPara
   pa.rmax_f = rmax_f; pa.undirected = prm.undirected; pa.vmark = vmark;
   pa.hub_deg = prm.hub_degree;
   pa.co_f = prm.cofrac >= 1.0 ? rmax_f : (float)(prm.rmax * std::max(prm.cofrac, 0.0));
+  pa.cap = P.cap;
   pa.heavy_w = P.heavy_w; pa.heavy_item = P.heavy_item;
   pa.heavy_count = P.counters + 2; pa.heavy_cap = P.heavy_cap;
   pa.units = P.units; pa.unit_count = P.counters + 3; pa.unit_cap = P.unit_cap;
@@ -553,12 +660,16 @@ tsvd_status job_begin(PushJob &J, PprState &P, const Adjacency &A, const PprPara
   ca.nsrc = P.nsrc; ca.sp = P.sp; ca.r = P.r; ca.deg = A.deg; ca.rmax_f = rmax_f;
   ca.cap = P.cap; ca.overflow = P.counters + 4;
   ca.hub_deg = prm.hub_degree;
-  J.gpush = grid_for((int64_t)1 << 30, 256, 8);
-  J.gcol = grid_for(ceil_div(P.nwords, 64) * 256, 256, 8);
+  ca.light = light_degree(P);
+  ca.round = P.counters + 2; ca.clock = P.stats + kStatSlots * 4;
+  static const int push_resident = resident_blocks((const void *)push_kernel);
+  static const int heavy_resident = resident_blocks((const void *)push_heavy_kernel);
+  J.gpush = push_resident;
+  J.gheavy = heavy_resident;
+  J.gcol = collect_grid(P.nwords, &ca.words);
   J.level = std::max(1, prm.levels) - 1;
   J.done = false;
   J.rounds = 0;
-  J.kernel_ms = 0;
   return TSVD_OK;
 }
 
@@ -571,69 +682,135 @@ float level_theta(const PprParams &prm, int level, float rmax_f) {
   return std::max(theta, rmax_f);
 }
 
-// Launches `count` rounds on the job's stream (asynchronous).
-tsvd_status job_rounds(PushJob &J, int count) {
-  PprState &P = *J.P;
-  cudaStream_t st = J.st;
-  for (int k = 0; k < count; ++k) {
-    const int cur = P.cur, nxt = 1 - P.cur;
-    J.pa.front = P.front[cur];
-    J.pa.front_count = P.counters + cur;
-    TSVD_CUDA(cudaMemsetAsync(P.counters + 2, 0, 2 * sizeof(int32_t), st));
-    TSVD_CUDA(cudaMemsetAsync(P.counters + nxt, 0, sizeof(int32_t), st));
-    TSVD_CUDA(cudaEventRecord(P.kev[2 * k], st));
-    push_kernel<<<J.gpush, 256, 0, st>>>(J.pa);
-    TSVD_LAUNCH_CHECK();
-    push_heavy_kernel<<<J.gpush, 256, 0, st>>>(J.pa);
-    TSVD_LAUNCH_CHECK();
-    TSVD_CUDA(cudaEventRecord(P.kev[2 * k + 1], st));
-    J.ca.next = P.front[nxt];
-    J.ca.next_count = P.counters + nxt;
-    collect_kernel<<<J.gcol, 256, 0, st>>>(J.ca);
-    TSVD_LAUNCH_CHECK();
-    P.cur = nxt;
-    ++J.rounds;
+}  // namespace
+
+constexpr int kRounds = 4;  // rounds launched together (even: the frontier lists end as they began)
+
+// The kernels of kRounds rounds as one graph launch: twelve separate launches
+// cost the host 60-120 us, more than the kernels of a small round. Its
+// parameters are set again when a push has others (grown adjacency, next
+// threshold level).
+struct RoundGraph {
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  cudaGraphNode_t node[3 * kRounds] = {};
+  PushArgs pa{};
+  CollectArgs ca{};
+};
+
+static void graph_free(RoundGraph *g) {
+  if (!g) return;
+  if (g->exec) cudaGraphExecDestroy(g->exec);
+  if (g->graph) cudaGraphDestroy(g->graph);
+  delete g;
+}
+
+namespace {
+
+// Parameters of node k (kernel k % 3 of round k / 3) for the job's arguments.
+struct RoundNode {
+  PushArgs pa;
+  CollectArgs ca;
+  void *arg;
+  cudaKernelNodeParams p{};
+  RoundNode(const PushJob &J, int k) : pa(J.pa), ca(J.ca) {
+    const PprState &P = *J.P;
+    const int cur = (k / 3) & 1, nxt = 1 - cur;
+    pa.front = P.front[cur];
+    pa.front_count = P.counters + cur;
+    ca.next = P.front[nxt];
+    ca.next_count = P.counters + nxt;
+    ca.spent = P.counters + cur;
+    const void *fn[3] = {(const void *)push_kernel, (const void *)push_heavy_kernel,
+                         (const void *)collect_kernel};
+    const int grid[3] = {J.gpush, J.gheavy, J.gcol};
+    arg = k % 3 == 2 ? (void *)&ca : (void *)&pa;
+    p.func = const_cast<void *>(fn[k % 3]);
+    p.gridDim = dim3((unsigned)grid[k % 3]);
+    p.blockDim = dim3(256);
+    p.kernelParams = &arg;
   }
-  TSVD_CUDA(cudaMemcpyAsync(P.host_counters, P.counters, 8 * sizeof(int32_t),
-                            cudaMemcpyDeviceToHost, st));
+  RoundNode(const RoundNode &) = delete;
+};
+
+// The job's graph with its current arguments.
+tsvd_status job_graph(PushJob &J) {
+  PprState &P = *J.P;
+  RoundGraph *&g = P.graph;
+  if (g && std::memcmp(&g->pa, &J.pa, sizeof(PushArgs)) == 0 &&
+      std::memcmp(&g->ca, &J.ca, sizeof(CollectArgs)) == 0)
+    return TSVD_OK;
+  if (!g) {
+    g = new (std::nothrow) RoundGraph;
+    if (!g) return fail(TSVD_ERR_OOM, "push: graph");
+    cudaError_t e = cudaGraphCreate(&g->graph, 0);
+    for (int k = 0; k < 3 * kRounds && e == cudaSuccess; ++k) {
+      RoundNode n(J, k);
+      e = cudaGraphAddKernelNode(&g->node[k], g->graph, k ? &g->node[k - 1] : nullptr, k ? 1 : 0,
+                                 &n.p);
+    }
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, g->graph, 0);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      graph_free(g);
+      g = nullptr;
+      return fail(TSVD_ERR_DEVICE, "push: graph: %s", cudaGetErrorString(e));
+    }
+  } else {
+    for (int k = 0; k < 3 * kRounds; ++k) {
+      RoundNode n(J, k);
+      TSVD_CUDA(cudaGraphExecKernelNodeSetParams(g->exec, g->node[k], &n.p));
+    }
+  }
+  g->pa = J.pa;
+  g->ca = J.ca;
   return TSVD_OK;
 }
 
-// Waits for the job's launched rounds; ends the level when its frontier is
-// empty, starting the next level (or finishing) as the schedule says.
-tsvd_status job_poll(PushJob &J, int count, const PprParams &prm) {
+// An interval: kRounds rounds launched together.
+// Launches one and the copy of the counters it leaves (asynchronous). The
+// kernels reset the counters themselves.
+tsvd_status job_interval(PushJob &J, int slot) {
   PprState &P = *J.P;
-  TSVD_CUDA(cudaStreamSynchronize(J.st));
-  for (int k = 0; k < count; ++k) {
-    float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, P.kev[2 * k], P.kev[2 * k + 1]) == cudaSuccess) J.kernel_ms += ms;
-  }
-  if (P.host_counters[4]) return fail(TSVD_ERR_STATE, "push: frontier buffer overflow");
-  if (P.host_counters[P.cur] != 0) {
-    if (J.rounds >= prm.max_rounds)
-      return fail(TSVD_ERR_TIMEOUT, "push: %lld rounds without convergence", (long long)J.rounds);
-    return TSVD_OK;
-  }
-  if (J.level == 0) {
-    J.done = true;
-    return TSVD_OK;
-  }
-  // the frontier of this level is empty: re-examine parked pairs at the next
+  TSVD_CUDA(cudaGraphLaunch(P.graph->exec, J.st));
+  for (int k = 0; k < 3 * kRounds; ++k) count_launch();
+  TSVD_CUDA(cudaMemcpyAsync(P.host_counters + kCounters * slot, P.counters,
+                            kCounters * sizeof(int32_t), cudaMemcpyDeviceToHost, J.st));
+  TSVD_CUDA(cudaEventRecord(P.kev[slot], J.st));
+  return TSVD_OK;
+}
+
+// Waits for an interval; *empty: its frontier is.
+tsvd_status job_poll(PushJob &J, int slot, int64_t rounds, const PprParams &prm, bool *empty) {
+  PprState &P = *J.P;
+  TSVD_CUDA(cudaEventSynchronize(P.kev[slot]));
+  const int32_t *h = P.host_counters + kCounters * slot;
+  if (h[4]) return fail(TSVD_ERR_STATE, "push: frontier buffer overflow");
+  *empty = h[0] == 0 && h[kHighCount] == 0;
+  if (!*empty && rounds >= prm.max_rounds)
+    return fail(TSVD_ERR_TIMEOUT, "push: %lld rounds without convergence", (long long)rounds);
+  return TSVD_OK;
+}
+
+// The frontier of this level is empty: re-examine parked pairs at the next.
+tsvd_status job_lower(PushJob &J, const PprParams &prm) {
+  PprState &P = *J.P;
   --J.level;
   J.pa.theta_f = J.ca.theta_f = level_theta(prm, J.level, J.pa.rmax_f);
   unpark_kernel<<<grid_for(P.nwords, 256, 8), 256, 0, J.st>>>(P.tflag, P.pend, P.nwords);
   TSVD_LAUNCH_CHECK();
-  TSVD_CUDA(cudaMemsetAsync(P.counters + P.cur, 0, sizeof(int32_t), J.st));
-  J.ca.next = P.front[P.cur];
-  J.ca.next_count = P.counters + P.cur;
-  collect_kernel<<<J.gcol, 256, 0, J.st>>>(J.ca);
+  CollectArgs ca = J.ca;
+  ca.next = P.front[0];
+  ca.next_count = P.counters;
+  ca.spent = nullptr;
+  collect_kernel<<<J.gcol, 256, 0, J.st>>>(ca);
   TSVD_LAUNCH_CHECK();
   return TSVD_OK;
 }
 
 tsvd_status job_finish(PushJob &J, PushStats *out) {
   PprState &P = *J.P;
-  unsigned long long slots[kStatSlots * 4], hs[4] = {0, 0, 0, 0};
+  unsigned long long slots[kStatSlots * 4 + 2], hs[4] = {0, 0, 0, 0};
   TSVD_CUDA(cudaMemcpyAsync(slots, P.stats, sizeof slots, cudaMemcpyDeviceToHost, J.st));
   TSVD_CUDA(cudaStreamSynchronize(J.st));
   for (int k = 0; k < kStatSlots * 4; ++k) hs[k % 4] += slots[k];
@@ -643,7 +820,7 @@ tsvd_status job_finish(PushJob &J, PushStats *out) {
     out->edge_updates = (int64_t)hs[1];
     out->items = (int64_t)hs[2];
     out->item_edges = (int64_t)hs[3];
-    out->kernel_ms = J.kernel_ms;
+    out->kernel_ms = slots[kStatSlots * 4 + 1] * 1e-6;
   }
   P.seeded = false;
   return TSVD_OK;
@@ -656,10 +833,24 @@ tsvd_status ppr_push(PprState &P, const Adjacency &A, const PprParams &prm, uint
   PushJob J;
   TSVD_TRY(job_begin(J, P, A, prm, vmark, st));
   J.pa.theta_f = J.ca.theta_f = level_theta(prm, J.level, J.pa.rmax_f);
-  const int check_every = std::min(8, prm.check_every > 0 ? prm.check_every : 4);
+  // The host looks at an interval's frontier while the next interval runs, so
+  // the GPU does not wait for it; rounds with an empty frontier cost 6 us each.
   while (!J.done) {
-    TSVD_TRY(job_rounds(J, check_every));
-    TSVD_TRY(job_poll(J, check_every, prm));
+    TSVD_TRY(job_graph(J));
+    int slot = 0;
+    TSVD_TRY(job_interval(J, slot));
+    for (;;) {
+      TSVD_TRY(job_interval(J, 1 - slot));
+      J.rounds += kRounds;
+      bool empty = false;
+      TSVD_TRY(job_poll(J, slot, J.rounds, prm, &empty));
+      if (empty) break;
+      slot = 1 - slot;
+    }
+    if (J.level == 0)
+      J.done = true;
+    else
+      TSVD_TRY(job_lower(J, prm));
   }
   return job_finish(J, out);
 }
