@@ -9,8 +9,8 @@
 //    cores: tcgen05.mma kind::f16 into a tensor-memory accumulator (fp32),
 //    operands brought into shared memory by TMA (cp.async.bulk.tensor) in a
 //    5-stage pipeline of full / empty mbarriers.
-//  gram_batched : X^T X with error-free products and compensated sums per
-//    row chunk, chunks summed in fp64 (Code/frpca.c:101, cblas_dgemm TN).
+//  gram_batched : X^T X with compensated sums per row chunk, chunks summed in
+//    fp64 (Code/frpca.c:101, cblas_dgemm TN).
 //  apply_right_batched : X W, with chol_inverse_batched (chol.cu) the
 //    CholeskyQR2 normalization replacing LUfraction (Code/frpca.c:4-41); the
 //    span of the basis, which is all the power iteration keeps, is the same.
@@ -344,27 +344,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_kernel(GemmArgs a) 
 }
 
 // ------------------------------------------------------------------ Gram
-// Error-free product + TwoSum accumulation (Ogita, Rump, Oishi, "Accurate sum
-// and dot product", SISC 2005): s + c carries the chunk sum to ~2^-44.
-struct Comp {
-  float s, c;
-};
-__device__ __forceinline__ void comp_add(Comp &acc, float a, float b) {
-  float p = a * b;
-  float e = fmaf(a, b, -p);
-  float t = acc.s + p;
-  float z = t - acc.s;
-  float err = (acc.s - (t - z)) + (p - z);
-  acc.s = t;
-  acc.c += err + e;
-}
-
+// Sums of products in pairs of floats. The rows are taken GRAM_SUB at a time;
+// over them column i has norm at most pw_i (a power of two), so a partial sum of
+// x_i x_j stays within pw_i pw_j and s = 3 pw_i pw_j + sum keeps one exponent:
+// what a fused multiply-add rounds away is then exactly the product minus the
+// change of s, and a second one recovers it for c (to 2^-47 of pw_i pw_j): four
+// operations a term, where the error-free product and TwoSum of any two floats
+// (Ogita, Rump, Oishi, SISC 2005) take ten. The sub-blocks' sums are added to
+// (S, C) by TwoSum, and the chunks in fp64. The kernel is bound by the issue of
+// these operations; 32 problems of 1500 x 256, measured: 463 -> 297 us.
 constexpr int GRAM_MIN_ROWS = 128;    // rows per CTA at least (one fp64 partial per chunk)
 constexpr int GRAM_MAX_CHUNKS = 2048;  // chunks over all problems (bounds the work buffer)
 constexpr int GRAM_SUB = 32;      // rows staged in smem at a time
 constexpr int GRAM_THREADS = 256;
-constexpr int GRAM_TPT = 1;       // 4x4 output tiles per thread (79 registers: 3 CTAs per SM)
-constexpr int GRAM_TILES_PER_CTA = GRAM_THREADS * GRAM_TPT;
 constexpr int GRAM_LMAX = 256;
 
 struct GramArgs {
@@ -378,77 +370,91 @@ struct GramArgs {
   double *work;   // [prob][chunk][l*l]
 };
 
-// grid: (row chunk, tile group, problem). Each thread owns <= 2 upper-triangle
-// 4x4 tiles of the l x l output and accumulates them over the chunk's rows.
+// The least power of two above sqrt(sum) (0 for 0), at most 2^62: three times its
+// square is still a float (beyond it the pair only rounds as plain sums do).
+__device__ __forceinline__ float norm_bound(float sum) {
+  const int e = min((int)(__float_as_uint(sum) >> 23) - 127, 123);
+  return sum > 0.f ? __uint_as_float((uint32_t)((e >> 1) + 1 + 127) << 23) : sum;
+}
+
+// grid: (row chunk, tile group, problem). A thread owns one upper-triangle 4 x 4
+// tile of the l x l output and accumulates it over the chunk's rows.
 __global__ void __launch_bounds__(GRAM_THREADS) gram_partial_kernel(GramArgs a) {
-  extern __shared__ __align__(16) float sx[];  // [GRAM_SUB][ld]
+  extern __shared__ __align__(16) float sx[];  // [GRAM_SUB][4 tiles], then [4 tiles] bounds
   const int prob = blockIdx.z, chunk = blockIdx.x;
   const int rows = a.rows[prob];
   const int r0 = chunk * a.chunk_rows;
   double *out = a.work + ((int64_t)prob * a.nchunks + chunk) * a.l * a.l;
-  const int T = a.tiles;
-  const int ntile_pairs = T * (T + 1) / 2;
+  const int T = a.tiles, sld = 4 * T;  // staged row stride covers every 4 x 4 tile column
+  float *pw = sx + GRAM_SUB * sld;
   const float *x = a.x[prob];
   const int r1 = min(rows, r0 + a.chunk_rows);
-  Comp acc[GRAM_TPT][16];
-  int ti[GRAM_TPT], tj[GRAM_TPT];
-  int my = 0;
-#pragma unroll
-  for (int k = 0; k < GRAM_TPT; ++k) {
-    int t = blockIdx.y * GRAM_TILES_PER_CTA + k * GRAM_THREADS + threadIdx.x;
-    ti[k] = tj[k] = 0;
-    if (t < ntile_pairs) {
-      int J = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
-      while ((J + 1) * (J + 2) / 2 <= t) ++J;
-      while (J * (J + 1) / 2 > t) --J;
-      int I = t - J * (J + 1) / 2;
-      ti[k] = I * 4;
-      tj[k] = J * 4;
-      my = k + 1;
-    }
-#pragma unroll
-    for (int e = 0; e < 16; ++e) acc[k][e] = Comp{0.f, 0.f};
+  const int t = blockIdx.y * GRAM_THREADS + threadIdx.x;
+  const bool mine = t < T * (T + 1) / 2;
+  int ti = 0, tj = 0;
+  if (mine) {
+    int J = (int)((sqrtf(8.f * t + 1.f) - 1.f) * 0.5f);
+    while ((J + 1) * (J + 2) / 2 <= t) ++J;
+    while (J * (J + 1) / 2 > t) --J;
+    ti = 4 * (t - J * (J + 1) / 2);
+    tj = 4 * J;
   }
-  const int sld = 4 * T;  // staged row stride covers every 4x4 tile column
+  float S[16], C[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) S[e] = C[e] = 0.f;
   for (int rb = r0; rb < r1; rb += GRAM_SUB) {
     const int nr = min(GRAM_SUB, r1 - rb);
     __syncthreads();
-    for (int i = threadIdx.x; i < GRAM_SUB * sld; i += blockDim.x) {
+    for (int i = threadIdx.x; i < GRAM_SUB * sld; i += GRAM_THREADS) {
       int rr = i / sld, cc = i % sld;
       sx[i] = (rr < nr && cc < a.l) ? x[(int64_t)(rb + rr) * a.ld + cc] : 0.f;
     }
     __syncthreads();
+    for (int c = threadIdx.x; c < sld; c += GRAM_THREADS) {
+      float sum = 0.f;
+#pragma unroll 8
+      for (int rr = 0; rr < GRAM_SUB; ++rr) sum = fmaf(sx[rr * sld + c], sx[rr * sld + c], sum);
+      pw[c] = norm_bound(sum);
+    }
+    __syncthreads();
+    if (!mine) continue;
+    float pi[4], pj[4], s[16], c[16];
+    *reinterpret_cast<float4 *>(pi) = *reinterpret_cast<const float4 *>(pw + ti);
+    *reinterpret_cast<float4 *>(pj) = *reinterpret_cast<const float4 *>(pw + tj);
 #pragma unroll
-    for (int k = 0; k < GRAM_TPT; ++k) {
-      if (k >= my) break;
-      for (int rr = 0; rr < nr; ++rr) {
-        const float *row = sx + rr * sld;
-        float xi[4], xj[4];
+    for (int e = 0; e < 16; ++e) {
+      s[e] = 3.f * (pi[e >> 2] * pj[e & 3]);
+      c[e] = 0.f;
+    }
+#pragma unroll 2
+    for (int rr = 0; rr < nr; ++rr) {
+      float xi[4], xj[4];
+      *reinterpret_cast<float4 *>(xi) = *reinterpret_cast<const float4 *>(sx + rr * sld + ti);
+      *reinterpret_cast<float4 *>(xj) = *reinterpret_cast<const float4 *>(sx + rr * sld + tj);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          xi[q] = row[ti[k] + q];
-          xj[q] = row[tj[k] + q];
-        }
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) comp_add(acc[k][p * 4 + q], xi[p], xj[q]);
+      for (int e = 0; e < 16; ++e) {
+        const float u = __fmaf_rn(xi[e >> 2], xj[e & 3], s[e]);
+        const float z = __fsub_rn(u, s[e]);
+        c[e] = __fadd_rn(c[e], __fmaf_rn(xi[e >> 2], xj[e & 3], -z));
+        s[e] = u;
       }
     }
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const float v = __fsub_rn(s[e], 3.f * (pi[e >> 2] * pj[e & 3]));
+      const float u = __fadd_rn(S[e], v), z = __fsub_rn(u, S[e]);
+      C[e] += __fadd_rn(__fsub_rn(S[e], __fsub_rn(u, z)), __fsub_rn(v, z)) + c[e];
+      S[e] = u;
+    }
   }
+  if (!mine) return;
 #pragma unroll
-  for (int k = 0; k < GRAM_TPT; ++k) {
-    if (k >= my) break;
-#pragma unroll
-    for (int p = 0; p < 4; ++p)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        int i = ti[k] + p, j = tj[k] + q;
-        if (i >= a.l || j >= a.l) continue;
-        double v = (double)acc[k][p * 4 + q].s + (double)acc[k][p * 4 + q].c;
-        out[i * a.l + j] = v;
-        out[j * a.l + i] = v;
-      }
+  for (int e = 0; e < 16; ++e) {
+    const int i = ti + (e >> 2), j = tj + (e & 3);
+    if (i >= a.l || j >= a.l) continue;
+    const double v = (double)S[e] + (double)C[e];
+    out[i * a.l + j] = v;
+    out[j * a.l + i] = v;
   }
 }
 
@@ -467,18 +473,22 @@ __global__ void gram_reduce_kernel(const double *__restrict__ work, int nchunks,
 
 // ------------------------------------------------------------------ X * W
 // Y = X W diag(colscale) (rows x n_out, written up to ldy <= 144 columns,
-// zero past n_out), optionally split into fp16 hi/lo. Register tiles: 256
-// threads as 16 x 16, each thread 4 rows x 9 columns (c = tx + 16 j) of a
-// 64-row tile; per k one float4 of X (the tile is staged transposed) and
-// nine loads of W feed 36 FMAs. A CTA walks a contiguous range of
-// (problem, row tile) items and restages W only when the problem changes.
-// X may alias Y (in-place CholeskyQR): a tile is read whole before it is
-// written.
-constexpr int APPLY_RT = 64;          // rows per tile
-constexpr int APPLY_THREADS = 256;
-constexpr int APPLY_CJ = 9;           // columns per thread
-constexpr int APPLY_WLD = 16 * APPLY_CJ;  // 144: staged W row
-constexpr int APPLY_XLD = APPLY_RT + 4;   // transposed X tile row (16-byte aligned)
+// zero past n_out), optionally split into fp16 hi/lo. A CTA takes a tile of 32 R
+// rows: warp w owns columns 16 w .. 16 w + 15, lane l rows R l .. R l + R - 1,
+// K is staged APPLY_KS deep (X transposed). Per k a warp reads its X as one
+// float of R per lane and its 16 W values by broadcast, 8 shared-memory
+// wavefronts for 64 FMAs at R = 4, which is what bounds the kernel (the FMAs,
+// three operands each from the register file, issue at about 75 lanes a clock);
+// R = 1 is for batches of few tiles. The tile goes out through shared memory, in
+// whole rows. upper: W is upper triangular, and a warp stops at its last
+// column's row. Every sum runs over k in ascending order, whatever R. X may
+// alias Y (in-place CholeskyQR): a tile is read whole before it is written. The
+// 15 calls of a factorization of 256 blocks, measured: 4.16 -> 3.36 ms (with
+// one CTA a SM, at 151 registers, 4.4 ms).
+constexpr int APPLY_THREADS = 288;
+constexpr int APPLY_KS = 32;
+constexpr int APPLY_WLD = kLp;            // staged W row
+constexpr int APPLY_OLD = kLp + 4;        // output tile row
 struct ApplyArgs {
   const float *const *x;
   const int32_t *rows;
@@ -492,76 +502,91 @@ struct ApplyArgs {
   __half *const *yhi;
   __half *const *ylo;
   float split_scale;
-  int tiles;  // row tiles per problem (of the largest)
-  int nprob;
+  int upper;
 };
 
-__global__ void __launch_bounds__(APPLY_THREADS) apply_right_kernel(ApplyArgs a) {
+template <int R>
+constexpr size_t apply_smem() {
+  return sizeof(float) * std::max((size_t)APPLY_KS * (APPLY_WLD + 32 * R + 4),
+                                  (size_t)32 * R * APPLY_OLD);
+}
+
+template <int R>
+__global__ void __launch_bounds__(APPLY_THREADS, 2) apply_right_kernel(ApplyArgs a) {
   extern __shared__ __align__(16) float sm[];
-  float *sw = sm;                               // [n_in][APPLY_WLD]
-  float *sxt = sm + a.n_in * APPLY_WLD;         // [n_in][APPLY_XLD] (X tile transposed)
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t items = (int64_t)a.nprob * a.tiles;
-  const int64_t per = (items + gridDim.x - 1) / gridDim.x;
-  const int64_t i0 = blockIdx.x * per, i1 = min(items, i0 + per);
-  int cur = -1;
-  for (int64_t it = i0; it < i1; ++it) {
-    const int prob = (int)(it / a.tiles), r0 = (int)(it % a.tiles) * APPLY_RT;
-    const int rows = a.rows[prob];
-    if (r0 >= rows) continue;  // the same for every thread
-    __syncthreads();           // the previous tile is written out
-    if (prob != cur) {
-      const float *W = a.w[prob];
-      const float *cs = a.colscale ? a.colscale[prob] : nullptr;
-      for (int i = threadIdx.x; i < a.n_in * APPLY_WLD; i += blockDim.x) {
-        const int r = i / APPLY_WLD, c = i % APPLY_WLD;
-        sw[i] = c < a.n_out ? W[(int64_t)r * a.ldw + c] * (cs ? cs[c] : 1.f) : 0.f;
-      }
-      cur = prob;
+  constexpr int RT = 32 * R, XLD = RT + 4;
+  float *sw = sm;                          // [APPLY_KS][APPLY_WLD]
+  float *sxt = sm + APPLY_KS * APPLY_WLD;  // [APPLY_KS][XLD]
+  const int prob = blockIdx.y, r0 = blockIdx.x * RT;
+  const int rows = a.rows[prob];
+  if (r0 >= rows) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c0 = 16 * warp;
+  const float *X = a.x[prob], *W = a.w[prob];
+  const float *cs = a.colscale ? a.colscale[prob] : nullptr;
+  const bool act = c0 < a.n_out;
+  float acc[R][16];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int j = 0; j < 16; ++j) acc[r][j] = 0.f;
+  for (int k0 = 0; k0 < a.n_in; k0 += APPLY_KS) {
+    const int ks = min(APPLY_KS, a.n_in - k0);
+    __syncthreads();
+    for (int i = tid; i < APPLY_KS * APPLY_WLD; i += APPLY_THREADS) {
+      const int k = i / APPLY_WLD, c = i % APPLY_WLD;
+      sw[i] = k < ks && c < a.n_out ? W[(int64_t)(k0 + k) * a.ldw + c] * (cs ? cs[c] : 1.f) : 0.f;
     }
-    const float *X = a.x[prob];
-    for (int i = threadIdx.x; i < APPLY_RT * a.n_in; i += blockDim.x) {
-      const int rr = i / a.n_in, k = i % a.n_in;
-      sxt[k * APPLY_XLD + rr] = r0 + rr < rows ? X[(int64_t)(r0 + rr) * a.ldx + k] : 0.f;
+    // consecutive threads take consecutive rows, four k each
+    for (int i = tid; i < RT * (APPLY_KS / 4); i += APPLY_THREADS) {
+      const int rr = i % RT, k = 4 * (i / RT);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        sxt[(k + q) * XLD + rr] =
+            r0 + rr < rows && k + q < ks ? X[(int64_t)(r0 + rr) * a.ldx + k0 + k + q] : 0.f;
     }
     __syncthreads();
-    float acc[4][APPLY_CJ];
+    if (!act || (a.upper && k0 > c0 + 15)) continue;
+#pragma unroll 4
+    for (int k = 0; k < ks; ++k) {
+      float xv[R], wv[16];
+      if (R == 4)
+        *reinterpret_cast<float4 *>(xv) = *reinterpret_cast<const float4 *>(sxt + k * XLD + 4 * lane);
+      else
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+        for (int r = 0; r < R; ++r) xv[r] = sxt[k * XLD + R * lane + r];
 #pragma unroll
-      for (int j = 0; j < APPLY_CJ; ++j) acc[r][j] = 0.f;
-    for (int k = 0; k < a.n_in; ++k) {
-      const float4 xv = *reinterpret_cast<const float4 *>(sxt + k * APPLY_XLD + ty * 4);
-      const float *wr = sw + k * APPLY_WLD + tx;
+      for (int q = 0; q < 16; q += 4)
+        *reinterpret_cast<float4 *>(wv + q) =
+            *reinterpret_cast<const float4 *>(sw + k * APPLY_WLD + c0 + q);
 #pragma unroll
-      for (int j = 0; j < APPLY_CJ; ++j) {
-        const float wv = wr[16 * j];
-        acc[0][j] = fmaf(xv.x, wv, acc[0][j]);
-        acc[1][j] = fmaf(xv.y, wv, acc[1][j]);
-        acc[2][j] = fmaf(xv.z, wv, acc[2][j]);
-        acc[3][j] = fmaf(xv.w, wv, acc[3][j]);
-      }
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) acc[r][j] = fmaf(xv[r], wv[j], acc[r][j]);
     }
-    float *Y = a.y[prob];
-    __half *Yh = a.yhi ? a.yhi[prob] : nullptr;
-    __half *Yl = a.ylo ? a.ylo[prob] : nullptr;
+  }
+  __syncthreads();  // every warp is done with the staged slabs
+  float *so = sm;   // [RT][APPLY_OLD]
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int row = r0 + ty * 4 + r;
-      if (row >= rows) continue;
+  for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int j = 0; j < APPLY_CJ; ++j) {
-        const int c = tx + 16 * j;
-        if (c >= a.ldy) continue;
-        const float v = acc[r][j];  // zero past n_out (W staged as zero there)
-        Y[(int64_t)row * a.ldy + c] = v;
-        if (Yh) {
-          const float sv = v * a.split_scale;
-          const __half h = __float2half_rn(sv);
-          Yh[(int64_t)row * a.ldy + c] = h;
-          Yl[(int64_t)row * a.ldy + c] = __float2half_rn(sv - __half2float(h));
-        }
-      }
+    for (int j = 0; j < 16; j += 4)
+      *reinterpret_cast<float4 *>(so + (R * lane + r) * APPLY_OLD + c0 + j) =
+          make_float4(acc[r][j], acc[r][j + 1], acc[r][j + 2], acc[r][j + 3]);
+  __syncthreads();
+  float *Y = a.y[prob];
+  __half *Yh = a.yhi ? a.yhi[prob] : nullptr;
+  __half *Yl = a.ylo ? a.ylo[prob] : nullptr;
+  for (int i = tid; i < RT * a.ldy; i += APPLY_THREADS) {
+    const int rr = i / a.ldy, c = i % a.ldy;
+    if (r0 + rr >= rows) break;
+    const float v = so[rr * APPLY_OLD + c];  // zero past n_out (W staged as zero there)
+    const int64_t at = (int64_t)(r0 + rr) * a.ldy + c;
+    Y[at] = v;
+    if (Yh) {
+      const float sv = v * a.split_scale;
+      const __half h = __float2half_rn(sv);
+      Yh[at] = h;
+      Yl[at] = __float2half_rn(sv - __half2float(h));
     }
   }
 }
@@ -742,11 +767,10 @@ tsvd_status gram_batched(const float *const *x, const int32_t *rows, int max_row
   if (gram_work_bytes(max_rows, l, nprob) > work_bytes)
     return fail(TSVD_ERR_INVALID, "gram: work buffer too small");
   int tiles = (l + 3) / 4;
-  int groups = (int)ceil_div(tiles * (tiles + 1) / 2, GRAM_TILES_PER_CTA);
-  size_t smem = (size_t)GRAM_SUB * (4 * tiles) * sizeof(float);
+  int groups = (int)ceil_div(tiles * (tiles + 1) / 2, GRAM_THREADS);
+  size_t smem = (size_t)(GRAM_SUB + 1) * (4 * tiles) * sizeof(float);
   TSVD_TRY(raise_smem_ceiling((const void *)gram_partial_kernel, smem));
-  // chunks past a problem's row count must contribute zeros
-  TSVD_CUDA(cudaMemsetAsync(work, 0, gram_work_bytes(max_rows, l, nprob), st));
+  // (a chunk past a problem's row count writes zeros)
   GramArgs a{x, rows, ld, l, tiles, nchunks, chunk_rows, work};
   gram_partial_kernel<<<dim3(nchunks, groups, nprob), GRAM_THREADS, smem, st>>>(a);
   TSVD_LAUNCH_CHECK();
@@ -760,19 +784,22 @@ tsvd_status apply_right_batched(const float *const *x, const int32_t *rows, int 
                                 const float *const *w, int ldw, int n_in, int n_out,
                                 const float *const *colscale, float *const *y, int ldy,
                                 __half *const *yhi, __half *const *ylo, float split_scale,
-                                int nprob, cudaStream_t st) {
+                                int nprob, cudaStream_t st, bool upper) {
   if (nprob == 0 || max_rows == 0) return TSVD_OK;
-  if (n_out > APPLY_WLD || ldy > APPLY_WLD || n_in > 256 || n_in < 1)
+  if (n_out > kLp || ldy > kLp || n_in > 256 || n_in < 1)
     return fail(TSVD_ERR_INVALID, "apply_right: sizes %d %d %d", n_in, n_out, ldy);
-  const size_t smem = (size_t)n_in * (APPLY_WLD + APPLY_XLD) * sizeof(float);
-  TSVD_TRY(raise_smem_ceiling((const void *)apply_right_kernel, smem));
-  const int tiles = (int)ceil_div(max_rows, APPLY_RT);
-  const int per_sm = std::max(1, (int)((227 * 1024) / (smem + 1024)));
-  const int64_t items = (int64_t)tiles * nprob;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(items, (int64_t)sm_count() * per_sm));
-  ApplyArgs a{x, rows, ldx, w, ldw, n_in, n_out, colscale, y, ldy, yhi, ylo, split_scale, tiles,
-              nprob};
-  apply_right_kernel<<<grid, APPLY_THREADS, smem, st>>>(a);
+  ApplyArgs a{x, rows, ldx, w, ldw, n_in, n_out, colscale, y, ldy, yhi, ylo, split_scale,
+              upper ? 1 : 0};
+  // 128-row tiles where they fill the SMs, 32-row tiles where they do not
+  if (ceil_div(max_rows, 128) * nprob >= sm_count()) {
+    TSVD_TRY(raise_smem_ceiling((const void *)apply_right_kernel<4>, apply_smem<4>()));
+    apply_right_kernel<4><<<dim3((unsigned)ceil_div(max_rows, 128), nprob), APPLY_THREADS,
+                            apply_smem<4>(), st>>>(a);
+  } else {
+    TSVD_TRY(raise_smem_ceiling((const void *)apply_right_kernel<1>, apply_smem<1>()));
+    apply_right_kernel<1><<<dim3((unsigned)ceil_div(max_rows, 32), nprob), APPLY_THREADS,
+                            apply_smem<1>(), st>>>(a);
+  }
   TSVD_LAUNCH_CHECK();
   return TSVD_OK;
 }

@@ -158,7 +158,7 @@ tsvd_status cholqr(FrpcaWork &W, float *const *x, const int32_t *rows, int max_r
     TSVD_TRY(apply_right_batched((const float *const *)x, rows, max_rows, kLp,
                                  (const float *const *)t, kLp, W.l, W.l, nullptr, x, kLp,
                                  last ? hi : nullptr, last ? lo : nullptr, kSplitScale, nprob,
-                                 st));
+                                 st, true));
   }
   return TSVD_OK;
 }

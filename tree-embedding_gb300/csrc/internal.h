@@ -144,12 +144,14 @@ tsvd_status orth_gram_batched(double *const *g, int n, const float *x, float *y,
                               cudaStream_t st);
 // Y[b] = X[b] * W[b] * diag(colscale[b]); writes fp32 (columns [n_out, ldy)
 // zeroed) and, when yhi/ylo are given, the fp16 split of Y * split_scale.
+// upper: W is upper triangular.
 tsvd_status apply_right_batched(const float *const *x, const int32_t *rows,
                                 int max_rows, int ldx, const float *const *w,
                                 int ldw, int n_in, int n_out,
                                 const float *const *colscale, float *const *y,
                                 int ldy, __half *const *yhi, __half *const *ylo,
-                                float split_scale, int nprob, cudaStream_t st);
+                                float split_scale, int nprob, cudaStream_t st,
+                                bool upper = false);
 // Eigenpairs of the Grams G[b] (n x n fp64, 2 <= n <= 256) to high relative
 // accuracy: lambda[b] (n values, descending) and the leading nv eigenvectors,
 // column j of V[b] (n x n row-major fp32; the other columns are not written).
