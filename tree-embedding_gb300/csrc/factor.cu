@@ -16,6 +16,7 @@
 // root keeps U sqrt(S) = M V_d S^-1/2 (NC) or U = M V_d S^-1 (LP).
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 
 #include "factor.h"
 #include "philox_gauss.h"
@@ -180,67 +181,91 @@ __global__ void lp_split_kernel(const float *__restrict__ u, int nsrc, int d, in
 }  // namespace
 
 tsvd_status frpca_work_alloc(FrpcaWork &W, int nmax, int64_t rows_max, int sp, int l, int d,
-                             bool direct) {
+                             bool direct, DeviceArena *arena, cudaStream_t st) {
+  const bool count = arena && arena->count;
   W.nmax = nmax;
   W.direct = direct;
+  W.in_arena = arena != nullptr;
   W.rows_max = std::max<int64_t>(rows_max, 1);
   W.sp = sp;
   W.l = l;
   W.d = d;
   size_t rk = (size_t)nmax * W.rows_max * kLp;
   size_t sk = (size_t)nmax * sp * kLp;
-  TSVD_CUDA(cudaMalloc(&W.xhi, rk * sizeof(__half)));
-  TSVD_CUDA(cudaMalloc(&W.xlo, rk * sizeof(__half)));
-  TSVD_CUDA(cudaMalloc(&W.z, std::max(rk, (size_t)nmax * sp * 256) * sizeof(float)));
-  TSVD_CUDA(cudaMalloc(&W.y, sk * sizeof(float)));
-  TSVD_CUDA(cudaMalloc(&W.qhi, sk * sizeof(__half)));
-  TSVD_CUDA(cudaMalloc(&W.qlo, sk * sizeof(__half)));
-  TSVD_CUDA(cudaMalloc(&W.g, (size_t)nmax * 256 * 256 * sizeof(double)));
-  TSVD_CUDA(cudaMalloc(&W.t, (size_t)nmax * kLp * kLp * sizeof(float)));
-  TSVD_CUDA(cudaMalloc(&W.lambda, (size_t)nmax * 256 * sizeof(float)));
-  TSVD_CUDA(cudaMalloc(&W.v, (size_t)nmax * 256 * 256 * sizeof(float)));
-  TSVD_CUDA(cudaMalloc(&W.colscale, (size_t)nmax * 2 * 256 * sizeof(float)));
-  TSVD_CUDA(cudaMalloc(&W.sums, (size_t)nmax * sizeof(double)));
+  TSVD_TRY(device_take(arena, &W.xhi, rk));
+  TSVD_TRY(device_take(arena, &W.xlo, rk));
+  TSVD_TRY(device_take(arena, &W.z, std::max(rk, (size_t)nmax * sp * 256)));
+  TSVD_TRY(device_take(arena, &W.y, sk));
+  TSVD_TRY(device_take(arena, &W.qhi, sk));
+  TSVD_TRY(device_take(arena, &W.qlo, sk));
+  TSVD_TRY(device_take(arena, &W.g, (size_t)nmax * 256 * 256));
+  TSVD_TRY(device_take(arena, &W.t, (size_t)nmax * kLp * kLp));
+  TSVD_TRY(device_take(arena, &W.lambda, (size_t)nmax * 256));
+  TSVD_TRY(device_take(arena, &W.v, (size_t)nmax * 256 * 256));
+  TSVD_TRY(device_take(arena, &W.colscale, (size_t)nmax * 2 * 256));
+  TSVD_TRY(device_take(arena, &W.sums, (size_t)nmax));
   {
     // every batched Gram uses at most min(nprob * rows/128, 2048) row chunks
     const int64_t rows = std::max<int64_t>(W.rows_max, sp);
     const int64_t chunks = std::min<int64_t>((int64_t)nmax * ceil_div(rows, 128), 2048) + nmax;
     W.gram_bytes = (size_t)chunks * 256 * 256 * sizeof(double);
   }
-  TSVD_CUDA(cudaMalloc(&W.gram_work, W.gram_bytes));
+  TSVD_TRY(device_take(arena, (char **)&W.gram_work, W.gram_bytes));
   W.eig_bytes = eig_work_bytes(256, nmax);
-  TSVD_CUDA(cudaMalloc(&W.eig_work, W.eig_bytes));
-  TSVD_CUDA(cudaMalloc(&W.eig_stat, sizeof(int32_t)));
-  TSVD_CUDA(cudaMemset(W.eig_stat, 0, sizeof(int32_t)));
+  TSVD_TRY(device_take(arena, (char **)&W.eig_work, W.eig_bytes));
+  TSVD_TRY(device_take(arena, &W.eig_stat, 1));
+  if (!count) TSVD_CUDA(cudaMemsetAsync(W.eig_stat, 0, sizeof(int32_t), st));
+  W.ptr_slots = (size_t)nmax * 64 + 256;
+  TSVD_TRY(device_take(arena, &W.dptr, W.ptr_slots));
+  TSVD_TRY(device_take(arena, &W.dint, W.ptr_slots));
+  W.tmap_slots = (size_t)nmax * 6;
+  TSVD_TRY(device_take(arena, &W.tmap_dev, W.tmap_slots));
   if (direct) {
     W.jac_bytes = std::max(jacobi_work_bytes(256, nmax), jacobi_work_bytes(l, nmax));
-    TSVD_CUDA(cudaMalloc(&W.jac_work, W.jac_bytes));
+    TSVD_TRY(device_take(arena, (char **)&W.jac_work, W.jac_bytes));
     for (double **p : {&W.dv, &W.dt, &W.dh})
-      TSVD_CUDA(cudaMalloc(p, (size_t)nmax * 256 * 256 * sizeof(double)));
-    std::vector<double *> hp(nmax);
-    for (int i = 0; i < nmax; ++i) hp[i] = W.dh + (int64_t)i * 256 * 256;
-    TSVD_CUDA(cudaMalloc(&W.dh_ptrs, sizeof(double *) * nmax));
-    TSVD_CUDA(cudaMemcpy(W.dh_ptrs, hp.data(), sizeof(double *) * nmax, cudaMemcpyHostToDevice));
+      TSVD_TRY(device_take(arena, p, (size_t)nmax * 256 * 256));
+    TSVD_TRY(device_take(arena, &W.dh_ptrs, (size_t)nmax));
+    if (!count) {
+      std::vector<double *> hp(nmax);
+      for (int i = 0; i < nmax; ++i) hp[i] = W.dh + (int64_t)i * 256 * 256;
+      TSVD_CUDA(cudaMemcpyAsync(W.dh_ptrs, hp.data(), sizeof(double *) * nmax,
+                                cudaMemcpyHostToDevice, st));
+      TSVD_CUDA(cudaStreamSynchronize(st));
+    }
   }
-  W.ptr_slots = (size_t)nmax * 64 + 256;
-  TSVD_CUDA(cudaMalloc(&W.dptr, W.ptr_slots * sizeof(void *)));
+  if (count) return TSVD_OK;
+  if (arena) {
+    W.hptr = static_cast<void **>(std::malloc(W.ptr_slots * sizeof(void *)));
+    W.hint = static_cast<int32_t *>(std::malloc(W.ptr_slots * sizeof(int32_t)));
+    W.tmap_host = static_cast<CUtensorMap *>(
+        std::aligned_alloc(alignof(CUtensorMap), W.tmap_slots * sizeof(CUtensorMap)));
+    if (!W.hptr || !W.hint || !W.tmap_host) return fail(TSVD_ERR_OOM, "frpca: staging");
+    return TSVD_OK;
+  }
   TSVD_CUDA(cudaMallocHost(&W.hptr, W.ptr_slots * sizeof(void *)));
-  TSVD_CUDA(cudaMalloc(&W.dint, W.ptr_slots * sizeof(int32_t)));
   TSVD_CUDA(cudaMallocHost(&W.hint, W.ptr_slots * sizeof(int32_t)));
-  W.tmap_slots = (size_t)nmax * 6;
-  TSVD_CUDA(cudaMalloc(&W.tmap_dev, W.tmap_slots * sizeof(CUtensorMap)));
   TSVD_CUDA(cudaMallocHost(&W.tmap_host, W.tmap_slots * sizeof(CUtensorMap)));
+  TSVD_CUDA(cudaStreamSynchronize(st));
   return TSVD_OK;
 }
 
 void frpca_work_free(FrpcaWork &W) {
+  // the wide merge's buffers, allocated on first use
+  cudaFree(W.wm); cudaFree(W.wv); cudaFree(W.ww); cudaFree(W.wy); cudaFree(W.wy2);
+  cudaFree(W.wnorm); cudaFree(W.wk);
+  if (W.in_arena) {
+    std::free(W.hptr);
+    std::free(W.hint);
+    std::free(W.tmap_host);
+    W = FrpcaWork();
+    return;
+  }
   cudaFree(W.xhi); cudaFree(W.xlo); cudaFree(W.z); cudaFree(W.y); cudaFree(W.qhi);
   cudaFree(W.qlo); cudaFree(W.g); cudaFree(W.t); cudaFree(W.lambda); cudaFree(W.v);
   cudaFree(W.colscale); cudaFree(W.sums); cudaFree(W.gram_work); cudaFree(W.eig_work); cudaFree(W.eig_stat); cudaFree(W.dptr);
   cudaFreeHost(W.hptr); cudaFree(W.dint); cudaFreeHost(W.hint);
   cudaFree(W.tmap_dev); cudaFreeHost(W.tmap_host);
-  cudaFree(W.wm); cudaFree(W.wv); cudaFree(W.ww); cudaFree(W.wy); cudaFree(W.wy2);
-  cudaFree(W.wnorm); cudaFree(W.wk);
   cudaFree(W.jac_work); cudaFree(W.dv); cudaFree(W.dt); cudaFree(W.dh); cudaFree(W.dh_ptrs);
   cudaGetLastError();  // the launch checks read this slot: leave nothing from teardown in it
   W = FrpcaWork();
@@ -742,7 +767,7 @@ tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, 
 
 }  // namespace
 
-tsvd_status merge_matrix(FrpcaWork &W, const float *m_host, int rows, int cols, float *out,
+tsvd_status merge_matrix(FrpcaWork &W, const float *m, int rows, int cols, float *out,
                          float *sigma_out, cudaStream_t st) {
   if (rows > W.sp) return fail(TSVD_ERR_INVALID, "merge: %d rows > %d", rows, W.sp);
   MergeProblem prob{};
@@ -750,12 +775,10 @@ tsvd_status merge_matrix(FrpcaWork &W, const float *m_host, int rows, int cols, 
   prob.sigma_out = sigma_out;
   if (cols > 256) {
     TSVD_TRY(wide_reserve(W, 1, cols));
-    TSVD_CUDA(cudaMemcpyAsync(W.wm, m_host, sizeof(float) * rows * cols, cudaMemcpyHostToDevice,
-                              st));
+    TSVD_CUDA(cudaMemcpyAsync(W.wm, m, sizeof(float) * rows * cols, cudaMemcpyDeviceToDevice, st));
     return merge_wide_core(W, &prob, 1, cols, rows, 0, st);
   }
-  TSVD_CUDA(cudaMemcpyAsync(W.z, m_host, sizeof(float) * rows * cols, cudaMemcpyHostToDevice, st));
-  return merge_finish(W, &prob, 1, cols, rows, 0, std::vector<float *>{W.z}, st);
+  return merge_finish(W, &prob, 1, cols, rows, 0, std::vector<float *>{const_cast<float *>(m)}, st);
 }
 
 tsvd_status merge_batch(FrpcaWork &W, const MergeProblem *probs, int nprob, int h, int nsrc,

@@ -23,6 +23,7 @@ struct FrpcaWork {
   void *eig_work = nullptr;
   size_t eig_bytes = 0;
   bool direct = false;     // results go to a caller of tsvd_frpca* / tsvd_merge_svd
+  bool in_arena = false;   // buffers belong to the caller's DeviceArena
   void *jac_work = nullptr;  // the two-sided eigen-solve's buffers (direct only)
   size_t jac_bytes = 0;
   double *dv = nullptr, *dt = nullptr, *dh = nullptr;  // [nmax][256*256] its refinement
@@ -50,12 +51,24 @@ struct FrpcaWork {
   int wide_iters = 0;       // subspace iterations of the last wide merge level
 };
 
+// Carves buffers out of one allocation (256-byte steps); with count set it only
+// adds up what they take.
+struct DeviceArena {
+  char *base = nullptr;
+  size_t used = 0, cap = 0;
+  bool count = false;
+};
+
 // Direct eigen-solves of up to this many columns take the one-sided solver:
 // there its results and the two-sided one's agree to 1e-5 (see jacobi.cu).
 constexpr int kDirectOneSided = 48;
 
+// arena: device buffers from it and staging from the heap, for a caller that
+// allocates once per call (frpca_work_free then frees the staging only);
+// otherwise every buffer on its own and pinned staging.
 tsvd_status frpca_work_alloc(FrpcaWork &W, int nmax, int64_t rows_max, int sp, int l, int d,
-                             bool direct = false);
+                             bool direct = false, DeviceArena *arena = nullptr,
+                             cudaStream_t st = nullptr);
 void frpca_work_free(FrpcaWork &W);
 tsvd_status eig_sweeps_fetch(FrpcaWork &W, cudaStream_t st);
 
@@ -82,6 +95,20 @@ struct FrpcaProblem {
 tsvd_status frpca_batch(FrpcaWork &W, const FrpcaProblem *probs, int nprob, int q,
                         uint64_t seed, int nsrc, cudaStream_t st, double *sum_sigma2);
 
+template <typename T>
+tsvd_status device_take(DeviceArena *A, T **p, size_t n) {
+  if (!A) {
+    TSVD_CUDA(cudaMalloc(p, n * sizeof(T)));
+    return TSVD_OK;
+  }
+  const size_t at = A->used;
+  A->used += (n * sizeof(T) + 255) & ~(size_t)255;
+  if (A->count) return TSVD_OK;
+  if (A->used > A->cap) return fail(TSVD_ERR_STATE, "arena of %zu bytes too small", A->cap);
+  *p = reinterpret_cast<T *>(A->base + at);
+  return TSVD_OK;
+}
+
 struct MergeProblem {
   const float *children[16];  // h child factors, |S| x d (ld d)
   float *out;                 // |S| x d (ld d)
@@ -90,10 +117,10 @@ struct MergeProblem {
 
 // Truncated SVD of [B_1 ... B_h] for every problem; out = U_d * diag(s_d) * f(s_d)
 // with f = 1 (inner node), s^-1/2 (root, U sqrt(S)) or s^-1 (root, U).
-// The merge of one ready matrix: m_host (rows x cols row-major fp32, host);
+// The merge of one ready matrix: m (rows x cols row-major fp32, device);
 // out (rows x d, device) = U_d diag(s_d), sigma_out (d, device) = s_d. W
 // sized by frpca_work_alloc with sp >= rows.
-tsvd_status merge_matrix(FrpcaWork &W, const float *m_host, int rows, int cols, float *out,
+tsvd_status merge_matrix(FrpcaWork &W, const float *m, int rows, int cols, float *out,
                          float *sigma_out, cudaStream_t st);
 
 tsvd_status merge_batch(FrpcaWork &W, const MergeProblem *probs, int nprob, int h, int nsrc,
