@@ -445,13 +445,15 @@ tsvd_status frpca_batch(FrpcaWork &W, const FrpcaProblem *probs, int nprob, int 
   auto prod_fwd = [&](const __half *const *hi, const __half *const *lo,
                       float scale) -> tsvd_status {
     if (sparse)
-      return spmm_batched(d_rptr, d_ridx, d_rval, d_sprows, sp, hi, lo, d_y, scale, nprob, st);
+      return spmm_batched(d_rptr, d_ridx, d_rval, d_sprows, sp, hi, lo, d_y, scale, l,
+                          nprob, st);
     return gemm_fwd(gb_fwd, lo != nullptr, d_y, W.y, ybytes, sp, max_nc, scale, st);
   };
   auto prod_bwd = [&](const __half *const *hi, const __half *const *lo,
                       float scale) -> tsvd_status {
     if (sparse)
-      return spmm_batched(d_cptr, d_cidx, d_cval, d_nc, max_nc, hi, lo, d_z, scale, nprob, st);
+      return spmm_batched(d_cptr, d_cidx, d_cval, d_nc, max_nc, hi, lo, d_z, scale, l,
+                          nprob, st);
     return gemm_bwd(gb_bwd, lo != nullptr, d_z, sp, max_nc, scale, st);
   };
   const int niter = (q - 1) / 2;

@@ -300,56 +300,148 @@ struct SpmmArgs {
   const __half *const *hi, *const *lo;
   float *const *y;
   float scale;
+  int l;    // columns of hi and lo that are not zero
+  int rpc;  // rows a CTA takes at a time (at most SPMM_WARPS)
+  int long_row;  // rows of more entries are the whole CTA's
 };
 
-// One warp per output row: lane l accumulates half2 columns l, l + 32 and
-// (lanes 0-7) l + 64 of the kLp = 144 wide row; the row's entries are read
-// 32 at a time by the lanes and broadcast.
-__global__ void __launch_bounds__(256) spmm_kernel(SpmmArgs a) {
+// A CTA takes a.rpc rows: one of up to a.long_row entries is a warp's, a longer
+// one all warps' together. A subgroup of LP lanes, eight columns (16 bytes of hi
+// and of lo) a lane, takes a contiguous part of the row, reads its entries by its
+// lanes and broadcasts them, with the loads of eight in flight before the first
+// is used; the subgroups' sums are added in a fixed order. Columns past l are zero
+// in the input and only written. The kernel is bound by the latency of its loads
+// along the longest row, and by L2 where there are many. Per product, measured
+// (before: a warp a row over all 144 columns, entry by entry): 600 x 3001 with 90k
+// entries in rows of very different length, l = 37, 168 -> 12 us, in equal rows
+// 15 to 64 -> 8 to 12 us; 1500 x 6000 with 900k entries, l = 133, 72 to 185 -> 37
+// to 66 us.
+constexpr int SPMM_WARPS = 8;
+
+// acc += N entries, whose columns and values lanes k .. k + N - 1 hold.
+template <int N, int LP, bool LO>
+__device__ __forceinline__ void spmm_entries(const uint4 *hi, const uint4 *lo, unsigned mask,
+                                             int32_t my_c, float my_v, int k, int piece,
+                                             float (&acc)[8]) {
+  uint4 h[N], w[N];
+  float v[N];
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    const int64_t at = (int64_t)__shfl_sync(mask, my_c, k + u, LP) * (kLp / 8) + piece;
+    v[u] = __shfl_sync(mask, my_v, k + u, LP);
+    h[u] = hi[at];
+    if (LO) w[u] = lo[at];
+  }
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    const __half2 *hp = reinterpret_cast<const __half2 *>(&h[u]);
+    const __half2 *wp = reinterpret_cast<const __half2 *>(&w[u]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float2 x = __half22float2(hp[j]);
+      if (LO) {
+        const float2 z = __half22float2(wp[j]);
+        x.x += z.x;
+        x.y += z.y;
+      }
+      acc[2 * j] = fmaf(v[u], x.x, acc[2 * j]);
+      acc[2 * j + 1] = fmaf(v[u], x.y, acc[2 * j + 1]);
+    }
+  }
+}
+
+// acc += the part of the entries [t0, t1) that subgroup g of n takes.
+template <int LP, bool LO>
+__device__ __forceinline__ void spmm_run(const int32_t *idx, const float *val, const uint4 *hi,
+                                         const uint4 *lo, int64_t t0, int64_t t1, int g, int n,
+                                         int piece, float (&acc)[8]) {
+  const int lane = threadIdx.x & 31, sl = lane & (LP - 1);
+  const unsigned mask = LP == 32 ? kFull : ((1u << LP) - 1u) << (lane & ~(LP - 1));
+  const int64_t part = ((t1 - t0 + n - 1) / n + 7) & ~(int64_t)7;
+  const int64_t tb0 = t0 + g * part, tb1 = tb0 + part < t1 ? tb0 + part : t1;
+  for (int64_t tb = tb0; tb < tb1; tb += LP) {
+    const int cnt = (int)(tb1 - tb < LP ? tb1 - tb : LP);
+    const int32_t my_c = sl < cnt ? idx[tb + sl] : 0;
+    const float my_v = sl < cnt ? val[tb + sl] : 0.f;
+    int k = 0;
+    for (; k + 8 <= cnt; k += 8)
+      spmm_entries<8, LP, LO>(hi, lo, mask, my_c, my_v, k, piece, acc);
+    if (k + 4 <= cnt) {
+      spmm_entries<4, LP, LO>(hi, lo, mask, my_c, my_v, k, piece, acc);
+      k += 4;
+    }
+    if (k + 2 <= cnt) {
+      spmm_entries<2, LP, LO>(hi, lo, mask, my_c, my_v, k, piece, acc);
+      k += 2;
+    }
+    if (k < cnt) spmm_entries<1, LP, LO>(hi, lo, mask, my_c, my_v, k, piece, acc);
+  }
+}
+
+template <int LP, bool LO>
+__global__ void __launch_bounds__(32 * SPMM_WARPS) spmm_kernel(SpmmArgs a) {
+  __shared__ __align__(16) float part[SPMM_WARPS][kLp];
+  constexpr int SUB = 32 / LP;  // subgroups of a warp
   const int prob = blockIdx.y;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int sl = lane & (LP - 1), sub = lane / LP;
   const int32_t rows = a.rows_out[prob];
   const int64_t *ptr = a.ptr[prob];
   const int32_t *idx = a.idx[prob];
   const float *val = a.val[prob];
-  const __half2 *hi = reinterpret_cast<const __half2 *>(a.hi[prob]);
-  const __half2 *lo = a.lo ? reinterpret_cast<const __half2 *>(a.lo[prob]) : nullptr;
-  float2 *y = reinterpret_cast<float2 *>(a.y[prob]);
-  constexpr int H = kLp / 2;  // 72 half2 per row
-  const bool third = lane + 64 < H;
-  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t r = gw; r < rows; r += nw) {
-    float2 acc0 = make_float2(0.f, 0.f), acc1 = acc0, acc2 = acc0;
-    const int64_t t0 = ptr[r], t1 = ptr[r + 1];
-    for (int64_t tb = t0; tb < t1; tb += 32) {
-      const int cnt = (int)(t1 - tb < 32 ? t1 - tb : 32);
-      const int32_t my_c = lane < cnt ? idx[tb + lane] : 0;
-      const float my_v = lane < cnt ? val[tb + lane] : 0.f;
-      for (int k = 0; k < cnt; ++k) {
-        const int64_t row = (int64_t)__shfl_sync(kFull, my_c, k) * H;
-        const float v = __shfl_sync(kFull, my_v, k);
-        float2 x0 = __half22float2(hi[row + lane]);
-        float2 x1 = __half22float2(hi[row + lane + 32]);
-        float2 x2 = third ? __half22float2(hi[row + lane + 64]) : make_float2(0.f, 0.f);
-        if (lo) {
-          const float2 l0 = __half22float2(lo[row + lane]);
-          const float2 l1 = __half22float2(lo[row + lane + 32]);
-          x0.x += l0.x; x0.y += l0.y; x1.x += l1.x; x1.y += l1.y;
-          if (third) {
-            const float2 l2 = __half22float2(lo[row + lane + 64]);
-            x2.x += l2.x; x2.y += l2.y;
-          }
+  const uint4 *hi = reinterpret_cast<const uint4 *>(a.hi[prob]);
+  const uint4 *lo = LO ? reinterpret_cast<const uint4 *>(a.lo[prob]) : nullptr;
+  float *y = a.y[prob];
+  const bool act = 8 * sl < a.l;
+  const int piece = act ? sl : 0;  // lanes past l repeat the first piece's loads
+  auto fold = [&](float (&acc)[8]) {  // the sum over the warp's subgroups, in each
+#pragma unroll
+    for (int o = LP; o < 32; o *= 2)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(kFull, acc[j], o);
+  };
+  for (int64_t r0 = (int64_t)blockIdx.x * a.rpc; r0 < rows; r0 += (int64_t)gridDim.x * a.rpc) {
+    const int nr = (int)(rows - r0 < a.rpc ? rows - r0 : a.rpc);
+    if (warp < nr) {
+      const int64_t r = r0 + warp, t0 = ptr[r], t1 = ptr[r + 1];
+      if (t1 - t0 <= a.long_row) {
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        spmm_run<LP, LO>(idx, val, hi, lo, t0, t1, sub, SUB, piece, acc);
+        __syncwarp();
+        fold(acc);
+        float4 *out = reinterpret_cast<float4 *>(y + r * kLp);
+        if (act && sub == 0) {
+          out[2 * sl] = make_float4(acc[0] * a.scale, acc[1] * a.scale, acc[2] * a.scale,
+                                    acc[3] * a.scale);
+          out[2 * sl + 1] = make_float4(acc[4] * a.scale, acc[5] * a.scale, acc[6] * a.scale,
+                                        acc[7] * a.scale);
         }
-        acc0.x = fmaf(v, x0.x, acc0.x); acc0.y = fmaf(v, x0.y, acc0.y);
-        acc1.x = fmaf(v, x1.x, acc1.x); acc1.y = fmaf(v, x1.y, acc1.y);
-        acc2.x = fmaf(v, x2.x, acc2.x); acc2.y = fmaf(v, x2.y, acc2.y);
+        for (int q = 2 * ((a.l + 7) / 8) + lane; q < kLp / 4; q += 32)
+          out[q] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
-    float2 *out = y + r * H;
-    out[lane] = make_float2(acc0.x * a.scale, acc0.y * a.scale);
-    out[lane + 32] = make_float2(acc1.x * a.scale, acc1.y * a.scale);
-    if (third) out[lane + 64] = make_float2(acc2.x * a.scale, acc2.y * a.scale);
+    for (int i = 0; i < nr; ++i) {  // the long rows
+      const int64_t r = r0 + i, t0 = ptr[r], t1 = ptr[r + 1];
+      if (t1 - t0 <= a.long_row) continue;
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      spmm_run<LP, LO>(idx, val, hi, lo, t0, t1, warp * SUB + sub, SPMM_WARPS * SUB, piece, acc);
+      __syncwarp();
+      fold(acc);
+      if (act && sub == 0) {
+        float4 *p = reinterpret_cast<float4 *>(part[warp] + 8 * sl);
+        p[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        p[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+      }
+      __syncthreads();
+      for (int c = threadIdx.x; c < kLp; c += 32 * SPMM_WARPS) {
+        float sum = 0.f;
+        if (c < a.l)
+#pragma unroll
+          for (int w = 0; w < SPMM_WARPS; ++w) sum += part[w][c];
+        y[r * kLp + c] = sum * a.scale;
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -607,12 +699,20 @@ tsvd_status plain_block_build(PlainBlockWork &W, const BlockSource &src, int64_t
 tsvd_status spmm_batched(const int64_t *const *ptr, const int32_t *const *idx,
                          const float *const *val, const int32_t *rows_out, int max_rows,
                          const __half *const *hi, const __half *const *lo, float *const *y,
-                         float scale, int nprob, cudaStream_t st) {
+                         float scale, int l, int nprob, cudaStream_t st) {
   if (nprob == 0 || max_rows == 0) return TSVD_OK;
-  SpmmArgs a{ptr, idx, val, rows_out, hi, lo, y, scale};
-  const int gx = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(max_rows, 8),
+  // Few rows: one a CTA, all its warps on it. Many: a warp each but for the
+  // longest (6000 rows of 150 entries: 256 us with the CTA on each from 64 entries
+  // on, 59 us so).
+  const int rpc = (int)std::max<int64_t>(
+      1, std::min<int64_t>(SPMM_WARPS, (int64_t)max_rows * nprob / (4 * sm_count())));
+  SpmmArgs a{ptr, idx, val, rows_out, hi, lo, y, scale, l, rpc, rpc == SPMM_WARPS ? 512 : 64};
+  const int gx = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(max_rows, rpc),
                                                              ceil_div(8ll * sm_count(), nprob)));
-  spmm_kernel<<<dim3(gx, nprob), 256, 0, st>>>(a);
+  auto *fn = l <= 64    ? (lo ? spmm_kernel<8, true> : spmm_kernel<8, false>)
+             : l <= 128 ? (lo ? spmm_kernel<16, true> : spmm_kernel<16, false>)
+                        : (lo ? spmm_kernel<32, true> : spmm_kernel<32, false>);
+  fn<<<dim3(gx, nprob), 32 * SPMM_WARPS, 0, st>>>(a);
   TSVD_LAUNCH_CHECK();
   return TSVD_OK;
 }

@@ -85,11 +85,11 @@ tsvd_status plain_block_build(PlainBlockWork &W, const BlockSource &src, int64_t
 void plain_block_free(PlainBlockWork &W);
 
 // Y[b] (rows_out x kLp fp32) = scale * S_b (rows_out x K, CSR) * (hi + lo)[b]
-// (K x kLp half, lo optional): the FP32 SpMM of the plain form, one warp per
-// output row, entries of a row summed in their stored order.
+// (K x kLp half, zero past column l, lo optional): the FP32 SpMM of the plain
+// form. Sums of a row in a fixed order.
 tsvd_status spmm_batched(const int64_t *const *ptr, const int32_t *const *idx,
                          const float *const *val, const int32_t *rows_out, int max_rows,
                          const __half *const *hi, const __half *const *lo, float *const *y,
-                         float scale, int nprob, cudaStream_t st);
+                         float scale, int l, int nprob, cudaStream_t st);
 
 }  // namespace tsvd
