@@ -555,28 +555,49 @@ tsvd_status merge_finish(FrpcaWork &W, const MergeProblem *probs, int nprob, int
   return TSVD_OK;
 }
 
-__global__ void colnorm_kernel(const float *__restrict__ m, int64_t nsrc, int n,
-                               float *__restrict__ norm) {
-  const int prob = blockIdx.y;
+// Squared norms of M's columns: 32 columns a CTA, their rows over its warps.
+__global__ void __launch_bounds__(1024) colnorm_kernel(const float *__restrict__ m, int64_t nsrc,
+                                                       int n, float *__restrict__ norm) {
+  __shared__ float part[32][33];
+  const int prob = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float *M = m + (int64_t)prob * nsrc * n;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-    float acc = 0.f;
-    for (int64_t s = 0; s < nsrc; ++s) acc = fmaf(M[s * n + c], M[s * n + c], acc);
-    norm[(int64_t)prob * n + c] = acc;
+  const int c = blockIdx.x * 32 + lane;
+  float acc = 0.f;
+  if (c < n)
+    for (int64_t s = warp; s < nsrc; s += 32) acc = fmaf(M[s * n + c], M[s * n + c], acc);
+  part[warp][lane] = acc;
+  __syncthreads();
+  if (warp == 0 && c < n) {
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) sum += part[w][lane];
+    norm[(int64_t)prob * n + c] = sum;
   }
 }
 
-// V[i] (n x p, row-major) = the columns sel[i][0..p) of the n x n identity.
-__global__ void select_basis_kernel(const int32_t *__restrict__ sel, int n, int p,
-                                    float *__restrict__ v) {
+// The p columns of the largest norms (of equal ones the first) to the front: V
+// (n x p, row-major, zero before) gets row c of the identity at c's rank.
+__global__ void __launch_bounds__(256) select_basis_kernel(const float *__restrict__ norm, int n,
+                                                           int p, float *__restrict__ v) {
+  extern __shared__ float nr[];
   const int prob = blockIdx.y;
-  float *V = v + (int64_t)prob * n * p;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < (int64_t)n * p;
-       i += (int64_t)gridDim.x * blockDim.x)
-    V[i] = 0.f;
+  for (int i = threadIdx.x; i < n; i += 256) nr[i] = norm[(int64_t)prob * n + i];
   __syncthreads();
-  if (blockIdx.x == 0)
-    for (int j = threadIdx.x; j < p; j += blockDim.x) V[(int64_t)sel[prob * p + j] * p + j] = 1.f;
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c >= n) return;
+  const float x = nr[c];
+  int rank = 0;
+  for (int i = 0; i < n; ++i) rank += nr[i] > x || (nr[i] == x && i < c);
+  if (rank < p) v[((int64_t)prob * n + c) * p + rank] = 1.f;
+}
+
+// out[i] = the trace of K[i] (l x l).
+__global__ void trace_kernel(const float *__restrict__ k, int l, double *__restrict__ out) {
+  const float *K = k + (int64_t)blockIdx.x * l * l;
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < l; i += 32) acc += (double)K[(int64_t)i * (l + 1)];
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (threadIdx.x == 0) out[blockIdx.x] = acc;
 }
 
 __global__ void diag_sum_kernel(double *const *g, int l, double *out) {
@@ -655,7 +676,7 @@ tsvd_status orthonormalize(FrpcaWork &W, float *x, int64_t xstride, float *y, in
 // and stopped when ||M V||_F^2 gains less than 1e-7 of itself. The result is
 // then the merge of the p columns of M V (compensated Gram + eigen-solve), the
 // same arithmetic as a narrow merge. The products are plain fp32 GEMMs
-// (sgemm_batched: fixed-order sums, 64 x 64 tiles).
+// (sgemm_batched: fixed-order sums).
 tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, int n, int nsrc,
                             int root_mode, cudaStream_t st);
 
@@ -695,36 +716,21 @@ tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, 
                          std::min(n, nsrc), d);
   const int64_t sm = (int64_t)nsrc * n, sv = (int64_t)n * p, sy = (int64_t)nsrc * p;
   // start: the p columns of M with the largest norms (the children's largest sigmas)
-  colnorm_kernel<<<dim3(ceil_div(n, 256), nprob), 256, 0, st>>>(W.wm, nsrc, n, W.wnorm);
+  colnorm_kernel<<<dim3((unsigned)ceil_div(n, 32), nprob), 1024, 0, st>>>(W.wm, nsrc, n, W.wnorm);
   TSVD_LAUNCH_CHECK();
-  std::vector<float> norms((size_t)nprob * n);
-  TSVD_CUDA(cudaMemcpyAsync(norms.data(), W.wnorm, sizeof(float) * norms.size(),
-                            cudaMemcpyDeviceToHost, st));
-  TSVD_CUDA(cudaStreamSynchronize(st));
-  std::vector<int32_t> sel((size_t)nprob * p);
-  for (int i = 0; i < nprob; ++i) {
-    std::vector<int32_t> idx(n);
-    for (int c = 0; c < n; ++c) idx[c] = c;
-    const float *nr = norms.data() + (size_t)i * n;
-    std::stable_sort(idx.begin(), idx.end(), [&](int32_t a, int32_t b) { return nr[a] > nr[b]; });
-    std::copy(idx.begin(), idx.begin() + p, sel.begin() + (size_t)i * p);
-  }
-  {
-    PtrPack pk(W);
-    const int32_t *d_sel = pk.add_int(sel);
-    TSVD_TRY(pk.upload(st));
-    select_basis_kernel<<<dim3(1, nprob), 256, 0, st>>>(d_sel, n, p, W.wv);
-    TSVD_LAUNCH_CHECK();
-    TSVD_CUDA(cudaStreamSynchronize(st));
-  }
+  TSVD_CUDA(cudaMemsetAsync(W.wv, 0, sizeof(float) * nprob * sv, st));
+  select_basis_kernel<<<dim3((unsigned)ceil_div(n, 256), nprob), 256, n * sizeof(float), st>>>(
+      W.wnorm, n, p, W.wv);
+  TSVD_LAUNCH_CHECK();
   std::vector<double> energy(nprob), prev(nprob, 0.0);
   // x (rows x p, row-major, problem stride xs) -> y: fp32 Gram (problem i at
   // W.wk + i p p), shifted fp32 Cholesky (factors after all the
   // Grams), triangular solve.
   const int64_t kp = (int64_t)p * p;
   auto cheap_basis = [&](const float *x, int64_t xs, float *y, int rows) -> tsvd_status {
-    // K = x^T x (p x p)
-    TSVD_TRY(sgemm_batched(true, p, p, rows, x, p, xs, x, p, xs, W.wk, p, kp, nprob, st));
+    // K = x^T x (p x p), its lower triangle
+    TSVD_TRY(sgemm_batched(true, p, p, rows, x, p, xs, x, p, xs, W.wk, p, kp, nprob, W.gram_work,
+                           W.gram_bytes, st, true));
     TSVD_TRY(chol_shift_solve_batched(W.wk, W.wk + nprob * kp, x, y, rows, p, xs, 1e-6f, nprob,
                                       st));
     return TSVD_OK;
@@ -732,26 +738,23 @@ tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, 
   int it = 0;
   for (; it < 40; ++it) {
     // Y = M V (|S| x p)
-    TSVD_TRY(sgemm_batched(false, nsrc, p, n, W.wm, n, sm, W.wv, p, sv, W.wy, p, sy, nprob, st));
+    TSVD_TRY(sgemm_batched(false, nsrc, p, n, W.wm, n, sm, W.wv, p, sv, W.wy, p, sy, nprob,
+                           W.gram_work, W.gram_bytes, st));
     TSVD_TRY(cheap_basis(W.wy, sy, W.wy2, nsrc));
     // ||M V||_F^2 = trace(Y^T Y), from the diagonal of the Gram just formed
-    std::vector<float> diag((size_t)nprob * p);
-    for (int i = 0; i < nprob; ++i)
-      TSVD_CUDA(cudaMemcpy2DAsync(diag.data() + (size_t)i * p, sizeof(float),
-                                  W.wk + i * kp, (p + 1) * sizeof(float), sizeof(float), p,
-                                  cudaMemcpyDeviceToHost, st));
+    trace_kernel<<<nprob, 32, 0, st>>>(W.wk, p, W.sums);
+    TSVD_LAUNCH_CHECK();
+    TSVD_CUDA(cudaMemcpyAsync(energy.data(), W.sums, sizeof(double) * nprob,
+                              cudaMemcpyDeviceToHost, st));
     TSVD_CUDA(cudaStreamSynchronize(st));
     bool done = it > 0;
-    for (int i = 0; i < nprob; ++i) {
-      double e = 0.0;
-      for (int j = 0; j < p; ++j) e += diag[(size_t)i * p + j];
-      energy[i] = e;
+    for (int i = 0; i < nprob; ++i)
       if (!(energy[i] - prev[i] <= 1e-6 * energy[i])) done = false;
-    }
     prev = energy;
     if (done) break;
     // W = M^T Yq (n x p)
-    TSVD_TRY(sgemm_batched(true, n, p, nsrc, W.wm, n, sm, W.wy2, p, sy, W.ww, p, sv, nprob, st));
+    TSVD_TRY(sgemm_batched(true, n, p, nsrc, W.wm, n, sm, W.wy2, p, sy, W.ww, p, sv, nprob,
+                           W.gram_work, W.gram_bytes, st));
     TSVD_TRY(cheap_basis(W.ww, sv, W.wv, n));
   }
   // one accurate CholeskyQR pass: an orthonormal V to working precision
@@ -763,7 +766,8 @@ tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, 
   std::vector<float *> z(nprob);
   for (int i = 0; i < nprob; ++i) z[i] = W.z + i * RK;
   // Z = M V (|S| x p), problem i at W.z + i RK
-  TSVD_TRY(sgemm_batched(false, nsrc, p, n, W.wm, n, sm, W.wv, p, sv, W.z, p, RK, nprob, st));
+  TSVD_TRY(sgemm_batched(false, nsrc, p, n, W.wm, n, sm, W.wv, p, sv, W.z, p, RK, nprob,
+                         W.gram_work, W.gram_bytes, st));
   return merge_finish(W, probs, nprob, p, nsrc, root_mode, z, st);
 }
 

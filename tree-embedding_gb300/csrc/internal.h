@@ -113,10 +113,13 @@ tsvd_status gemm_bwd(const GemmBatch &gb, bool has_lo, float *const *z, int sp, 
 tsvd_status gemm_check(cudaStream_t st);
 
 // C[z] = op(A[z]) B[z] in fp32, row-major (op(A) = A^T when trans_a: A is
-// K x M), problem z at z * stride of each operand; fixed-order sums.
+// K x M), problem z at z * stride of each operand; fixed-order sums. work holds
+// the partial sums where K is split over CTAs, as far as work_bytes allow.
+// lower: only the lower triangle of C is wanted.
 tsvd_status sgemm_batched(bool trans_a, int M, int N, int K, const float *A, int lda, int64_t sa,
                           const float *B, int ldb, int64_t sb, float *C, int ldc, int64_t sc,
-                          int nprob, cudaStream_t st);
+                          int nprob, void *work, size_t work_bytes, cudaStream_t st,
+                          bool lower = false);
 
 // G[b] (l x l fp64) = X[b]^T X[b], X row-major [rows_b][ld] fp32.
 tsvd_status gram_batched(const float *const *x, const int32_t *rows, int max_rows,
