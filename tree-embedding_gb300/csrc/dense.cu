@@ -353,7 +353,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_kernel(GemmArgs a) 
 // (Ogita, Rump, Oishi, SISC 2005) take ten. The sub-blocks' sums are added to
 // (S, C) by TwoSum, and the chunks in fp64. The kernel is bound by the issue of
 // these operations; 32 problems of 1500 x 256, measured: 463 -> 297 us.
-constexpr int GRAM_MIN_ROWS = 128;    // rows per CTA at least (one fp64 partial per chunk)
+constexpr int GRAM_MIN_ROWS = 128;    // rows per CTA (one fp64 partial per chunk); fewer
+                                      // where CTAs are few (gram_batched)
 constexpr int GRAM_MAX_CHUNKS = 2048;  // chunks over all problems (bounds the work buffer)
 constexpr int GRAM_SUB = 32;      // rows staged in smem at a time
 constexpr int GRAM_THREADS = 256;
@@ -451,23 +452,25 @@ __global__ void __launch_bounds__(GRAM_THREADS) gram_partial_kernel(GramArgs a) 
 #pragma unroll
   for (int e = 0; e < 16; ++e) {
     const int i = ti + (e >> 2), j = tj + (e & 3);
-    if (i >= a.l || j >= a.l) continue;
-    const double v = (double)S[e] + (double)C[e];
-    out[i * a.l + j] = v;
-    out[j * a.l + i] = v;
+    if (i < a.l && j < a.l) out[i * a.l + j] = (double)S[e] + (double)C[e];
   }
 }
 
+// Sums the chunks' upper 4 x 4 tiles and mirrors them.
 __global__ void gram_reduce_kernel(const double *__restrict__ work, int nchunks, int l,
                                    double *const *g, int nprob) {
   const int prob = blockIdx.y;
   const int64_t ll = (int64_t)l * l;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ll;
        i += (int64_t)gridDim.x * blockDim.x) {
+    const int r = (int)(i / l), c = (int)(i % l);
+    if (r / 4 > c / 4) continue;
     double s = 0.0;
     const double *w = work + (int64_t)prob * nchunks * ll + i;
-    for (int c = 0; c < nchunks; ++c) s += w[c * ll];
+#pragma unroll 8
+    for (int k = 0; k < nchunks; ++k) s += w[k * ll];
     g[prob][i] = s;
+    g[prob][(int64_t)c * l + r] = s;
   }
 }
 
@@ -768,6 +771,18 @@ tsvd_status gram_batched(const float *const *x, const int32_t *rows, int max_row
     return fail(TSVD_ERR_INVALID, "gram: work buffer too small");
   int tiles = (l + 3) / 4;
   int groups = (int)ceil_div(tiles * (tiles + 1) / 2, GRAM_THREADS);
+  // A slab of 32 rows is 3 us of a CTA's issue: halve the chunks until every SM has
+  // two, as far as the buffer goes (with the sum of the chunks, 1000 x 69, 4
+  // problems: 18 -> 11 us; 6000 x 133, one: 38 -> 30 us).
+  while (chunk_rows > GRAM_SUB && (int64_t)nchunks * groups * nprob < 2 * sm_count()) {
+    const int cr = (int)round_up(chunk_rows / 2, GRAM_SUB);
+    const int64_t nc = ceil_div(max_rows, cr);
+    if (cr == chunk_rows || nc * nprob > GRAM_MAX_CHUNKS ||
+        (size_t)(nc * nprob) * l * l * sizeof(double) > work_bytes)
+      break;
+    chunk_rows = cr;
+    nchunks = (int)nc;
+  }
   size_t smem = (size_t)(GRAM_SUB + 1) * (4 * tiles) * sizeof(float);
   TSVD_TRY(raise_smem_ceiling((const void *)gram_partial_kernel, smem));
   // (a chunk past a problem's row count writes zeros)
