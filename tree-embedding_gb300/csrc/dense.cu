@@ -477,17 +477,19 @@ __global__ void gram_reduce_kernel(const double *__restrict__ work, int nchunks,
 // ------------------------------------------------------------------ X * W
 // Y = X W diag(colscale) (rows x n_out, written up to ldy <= 144 columns,
 // zero past n_out), optionally split into fp16 hi/lo. A CTA takes a tile of 32 R
-// rows: warp w owns columns 16 w .. 16 w + 15, lane l rows R l .. R l + R - 1,
-// K is staged APPLY_KS deep (X transposed). Per k a warp reads its X as one
-// float of R per lane and its 16 W values by broadcast, 8 shared-memory
-// wavefronts for 64 FMAs at R = 4, which is what bounds the kernel (the FMAs,
-// three operands each from the register file, issue at about 75 lanes a clock);
-// R = 1 is for batches of few tiles. The tile goes out through shared memory, in
-// whole rows. upper: W is upper triangular, and a warp stops at its last
-// column's row. Every sum runs over k in ascending order, whatever R. X may
-// alias Y (in-place CholeskyQR): a tile is read whole before it is written. The
-// 15 calls of a factorization of 256 blocks, measured: 4.16 -> 3.36 ms (with
-// one CTA a SM, at 151 registers, 4.4 ms).
+// rows: warp w owns columns 16 w .. 16 w + 15, lane l rows l, l + 32, ..; K goes
+// APPLY_KS at a time through two stages of shared memory, the next slab of X and W
+// on its way (cp.async) while one is multiplied. Per four k a warp reads its X as
+// R float4 a lane and its 64 W values by broadcast, 32 shared-memory wavefronts for
+// 256 FMAs at R = 4, whose issue (three operands each from the register file, about
+// 75 lanes a clock) bounds large batches; small ones wait for their slabs, and take
+// R = 1. The tile goes out through shared memory, in whole rows of 16-byte stores.
+// upper: W is upper triangular, and a warp stops at its last column's row. Every
+// sum runs over k in ascending order, whatever R. X may alias Y (in-place
+// CholeskyQR): a tile is read whole before it is written. Measured, slabs fetched
+// between barriers and 4-byte stores before: 64 problems of 3125 x 133 (triangular,
+// with the split) 406 -> 205 us, 32 of 1500 x 256 208 -> 112, one of 1500 x 133 28
+// -> 13, of 1500 x 256 47 -> 20.
 constexpr int APPLY_THREADS = 288;
 constexpr int APPLY_KS = 32;
 constexpr int APPLY_WLD = kLp;            // staged W row
@@ -506,65 +508,94 @@ struct ApplyArgs {
   __half *const *ylo;
   float split_scale;
   int upper;
+  int vec;  // ldx and ldw are multiples of four
 };
 
+constexpr int APPLY_XLD = APPLY_KS + 4;   // staged X row
 template <int R>
 constexpr size_t apply_smem() {
-  return sizeof(float) * std::max((size_t)APPLY_KS * (APPLY_WLD + 32 * R + 4),
+  return sizeof(float) * std::max((size_t)2 * (32 * R * APPLY_XLD + APPLY_KS * APPLY_WLD),
                                   (size_t)32 * R * APPLY_OLD);
+}
+
+// BYTES (16 or 4) to shared memory, of which the first `in` come from src.
+template <int BYTES>
+__device__ __forceinline__ void cp_async_zfill(float *dst, const float *src, int in) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  if (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(in));
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(in));
+}
+
+// One slab (APPLY_KS deep, from k0) of X and W to shared memory, asynchronously; what
+// lies outside is zero. VEC: by 16 bytes (rows that begin on 16 bytes), else by 4.
+template <int R, bool VEC>
+__device__ __forceinline__ void apply_fetch(const ApplyArgs &a, const float *X, const float *W,
+                                            int r0, int rows, int k0, float *sx, float *sw) {
+  constexpr int V = VEC ? 4 : 1;
+  const int ks = min(APPLY_KS, a.n_in - k0);
+  for (int i = threadIdx.x; i < 32 * R * (APPLY_KS / V); i += APPLY_THREADS) {
+    const int k = V * (i % (APPLY_KS / V)), rr = i / (APPLY_KS / V);
+    const int in = r0 + rr < rows ? max(0, min(V, ks - k)) : 0;
+    cp_async_zfill<4 * V>(sx + rr * APPLY_XLD + k,
+                          in ? X + (int64_t)(r0 + rr) * a.ldx + k0 + k : X, 4 * in);
+  }
+  for (int i = threadIdx.x; i < APPLY_KS * (APPLY_WLD / V); i += APPLY_THREADS) {
+    const int c = V * (i % (APPLY_WLD / V)), k = i / (APPLY_WLD / V);
+    const int in = k < ks ? max(0, min(V, a.n_out - c)) : 0;
+    cp_async_zfill<4 * V>(sw + k * APPLY_WLD + c, in ? W + (int64_t)(k0 + k) * a.ldw + c : W,
+                          4 * in);
+  }
 }
 
 template <int R>
 __global__ void __launch_bounds__(APPLY_THREADS, 2) apply_right_kernel(ApplyArgs a) {
   extern __shared__ __align__(16) float sm[];
-  constexpr int RT = 32 * R, XLD = RT + 4;
-  float *sw = sm;                          // [APPLY_KS][APPLY_WLD]
-  float *sxt = sm + APPLY_KS * APPLY_WLD;  // [APPLY_KS][XLD]
+  constexpr int RT = 32 * R, STAGE = RT * APPLY_XLD + APPLY_KS * APPLY_WLD;
   const int prob = blockIdx.y, r0 = blockIdx.x * RT;
   const int rows = a.rows[prob];
   if (r0 >= rows) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c0 = 16 * warp;
   const float *X = a.x[prob], *W = a.w[prob];
-  const float *cs = a.colscale ? a.colscale[prob] : nullptr;
   const bool act = c0 < a.n_out;
   float acc[R][16];
 #pragma unroll
   for (int r = 0; r < R; ++r)
 #pragma unroll
     for (int j = 0; j < 16; ++j) acc[r][j] = 0.f;
-  for (int k0 = 0; k0 < a.n_in; k0 += APPLY_KS) {
-    const int ks = min(APPLY_KS, a.n_in - k0);
-    __syncthreads();
-    for (int i = tid; i < APPLY_KS * APPLY_WLD; i += APPLY_THREADS) {
-      const int k = i / APPLY_WLD, c = i % APPLY_WLD;
-      sw[i] = k < ks && c < a.n_out ? W[(int64_t)(k0 + k) * a.ldw + c] * (cs ? cs[c] : 1.f) : 0.f;
-    }
-    // consecutive threads take consecutive rows, four k each
-    for (int i = tid; i < RT * (APPLY_KS / 4); i += APPLY_THREADS) {
-      const int rr = i % RT, k = 4 * (i / RT);
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        sxt[(k + q) * XLD + rr] =
-            r0 + rr < rows && k + q < ks ? X[(int64_t)(r0 + rr) * a.ldx + k0 + k + q] : 0.f;
-    }
-    __syncthreads();
+  const bool vec = a.vec && (((uintptr_t)X | (uintptr_t)W) & 15) == 0;
+  auto fetch = [&](int k0, float *to) {
+    if (vec) apply_fetch<R, true>(a, X, W, r0, rows, k0, to, to + RT * APPLY_XLD);
+    else apply_fetch<R, false>(a, X, W, r0, rows, k0, to, to + RT * APPLY_XLD);
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  fetch(0, sm);
+  for (int k0 = 0, s = 0; k0 < a.n_in; k0 += APPLY_KS, s ^= 1) {
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();  // the slab is there, and every warp is done with the one before
+    if (k0 + APPLY_KS < a.n_in) fetch(k0 + APPLY_KS, sm + (s ^ 1) * STAGE);
     if (!act || (a.upper && k0 > c0 + 15)) continue;
-#pragma unroll 4
-    for (int k = 0; k < ks; ++k) {
-      float xv[R], wv[16];
-      if (R == 4)
-        *reinterpret_cast<float4 *>(xv) = *reinterpret_cast<const float4 *>(sxt + k * XLD + 4 * lane);
-      else
-#pragma unroll
-        for (int r = 0; r < R; ++r) xv[r] = sxt[k * XLD + R * lane + r];
-#pragma unroll
-      for (int q = 0; q < 16; q += 4)
-        *reinterpret_cast<float4 *>(wv + q) =
-            *reinterpret_cast<const float4 *>(sw + k * APPLY_WLD + c0 + q);
+    const float *sx = sm + s * STAGE + lane * APPLY_XLD, *sw = sm + s * STAGE + RT * APPLY_XLD + c0;
+    const int ks = min(APPLY_KS, a.n_in - k0);  // (what lies past it is zero)
+    for (int k = 0; k < ks; k += 4) {
+      float xv[R][4];
 #pragma unroll
       for (int r = 0; r < R; ++r)
+        *reinterpret_cast<float4 *>(xv[r]) =
+            *reinterpret_cast<const float4 *>(sx + 32 * r * APPLY_XLD + k);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[r][j] = fmaf(xv[r], wv[j], acc[r][j]);
+      for (int q = 0; q < 4; ++q) {
+        float wv[16];
+#pragma unroll
+        for (int j = 0; j < 16; j += 4)
+          *reinterpret_cast<float4 *>(wv + j) =
+              *reinterpret_cast<const float4 *>(sw + (k + q) * APPLY_WLD + j);
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) acc[r][j] = fmaf(xv[r][q], wv[j], acc[r][j]);
+      }
     }
   }
   __syncthreads();  // every warp is done with the staged slabs
@@ -573,24 +604,52 @@ __global__ void __launch_bounds__(APPLY_THREADS, 2) apply_right_kernel(ApplyArgs
   for (int r = 0; r < R; ++r)
 #pragma unroll
     for (int j = 0; j < 16; j += 4)
-      *reinterpret_cast<float4 *>(so + (R * lane + r) * APPLY_OLD + c0 + j) =
+      *reinterpret_cast<float4 *>(so + (lane + 32 * r) * APPLY_OLD + c0 + j) =
           make_float4(acc[r][j], acc[r][j + 1], acc[r][j + 2], acc[r][j + 3]);
   __syncthreads();
+  const float *cs = a.colscale ? a.colscale[prob] : nullptr;
   float *Y = a.y[prob];
   __half *Yh = a.yhi ? a.yhi[prob] : nullptr;
   __half *Yl = a.ylo ? a.ylo[prob] : nullptr;
+  auto split = [&](float v, __half &h, __half &l) {
+    const float sv = v * a.split_scale;
+    h = __float2half_rn(sv);
+    l = __float2half_rn(sv - __half2float(h));
+  };
+  // (columns past n_out are zero, as W was staged as zero there)
+  if (a.ldy % 4 == 0 && (((uintptr_t)Y | (uintptr_t)Yh | (uintptr_t)Yl) & 15) == 0) {
+    const int v4 = a.ldy / 4;
+    for (int i = tid; i < RT * v4; i += APPLY_THREADS) {
+      const int rr = i / v4, c = 4 * (i % v4);
+      if (r0 + rr >= rows) break;
+      float4 v = *reinterpret_cast<const float4 *>(so + rr * APPLY_OLD + c);
+      if (cs && c < a.n_out) {
+        v.x *= cs[c];
+        v.y *= c + 1 < a.n_out ? cs[c + 1] : 0.f;
+        v.z *= c + 2 < a.n_out ? cs[c + 2] : 0.f;
+        v.w *= c + 3 < a.n_out ? cs[c + 3] : 0.f;
+      }
+      const int64_t at = (int64_t)(r0 + rr) * a.ldy + c;
+      *reinterpret_cast<float4 *>(Y + at) = v;
+      if (Yh) {
+        __align__(8) __half h[4], l[4];
+        split(v.x, h[0], l[0]);
+        split(v.y, h[1], l[1]);
+        split(v.z, h[2], l[2]);
+        split(v.w, h[3], l[3]);
+        *reinterpret_cast<uint2 *>(Yh + at) = *reinterpret_cast<const uint2 *>(h);
+        *reinterpret_cast<uint2 *>(Yl + at) = *reinterpret_cast<const uint2 *>(l);
+      }
+    }
+    return;
+  }
   for (int i = tid; i < RT * a.ldy; i += APPLY_THREADS) {
     const int rr = i / a.ldy, c = i % a.ldy;
     if (r0 + rr >= rows) break;
-    const float v = so[rr * APPLY_OLD + c];  // zero past n_out (W staged as zero there)
+    const float v = so[rr * APPLY_OLD + c] * (cs && c < a.n_out ? cs[c] : 1.f);
     const int64_t at = (int64_t)(r0 + rr) * a.ldy + c;
     Y[at] = v;
-    if (Yh) {
-      const float sv = v * a.split_scale;
-      const __half h = __float2half_rn(sv);
-      Yh[at] = h;
-      Yl[at] = __float2half_rn(sv - __half2float(h));
-    }
+    if (Yh) split(v, Yh[at], Yl[at]);
   }
 }
 
@@ -804,7 +863,7 @@ tsvd_status apply_right_batched(const float *const *x, const int32_t *rows, int 
   if (n_out > kLp || ldy > kLp || n_in > 256 || n_in < 1)
     return fail(TSVD_ERR_INVALID, "apply_right: sizes %d %d %d", n_in, n_out, ldy);
   ApplyArgs a{x, rows, ldx, w, ldw, n_in, n_out, colscale, y, ldy, yhi, ylo, split_scale,
-              upper ? 1 : 0};
+              upper ? 1 : 0, ldx % 4 == 0 && ldw % 4 == 0 ? 1 : 0};
   // 128-row tiles where they fill the SMs, 32-row tiles where they do not
   if (ceil_div(max_rows, 128) * nprob >= sm_count()) {
     TSVD_TRY(raise_smem_ceiling((const void *)apply_right_kernel<4>, apply_smem<4>()));
