@@ -279,6 +279,12 @@ tsvd_status eig_sweeps_fetch(FrpcaWork &W, cudaStream_t st) {
   return TSVD_OK;
 }
 
+tsvd_status eig_check(const FrpcaWork &W) {
+  if (W.last_sweeps >= kEigTimedOut)
+    return fail(TSVD_ERR_TIMEOUT, "eigen-solve: a CTA gave up waiting for its cluster");
+  return TSVD_OK;
+}
+
 namespace {
 
 __global__ void widen_kernel(const float *__restrict__ v, double *__restrict__ out, int64_t count,
@@ -511,6 +517,7 @@ tsvd_status frpca_batch(FrpcaWork &W, const FrpcaProblem *probs, int nprob, int 
   TSVD_CUDA(cudaMemcpyAsync(hs.data(), d_sum2, sizeof(double) * nprob, cudaMemcpyDeviceToHost, st));
   TSVD_TRY(eig_sweeps_fetch(W, st));
   TSVD_CUDA(cudaStreamSynchronize(st));
+  TSVD_TRY(eig_check(W));
   if (sum_sigma2)
     for (int i = 0; i < nprob; ++i) sum_sigma2[i] = hs[i];
   return gemm_check(st);

@@ -71,6 +71,8 @@ tsvd_status frpca_work_alloc(FrpcaWork &W, int nmax, int64_t rows_max, int sp, i
                              cudaStream_t st = nullptr);
 void frpca_work_free(FrpcaWork &W);
 tsvd_status eig_sweeps_fetch(FrpcaWork &W, cudaStream_t st);
+// An error if a solve reported by the last fetch (st synchronized since) gave up.
+tsvd_status eig_check(const FrpcaWork &W);
 
 struct SparseBlock;
 

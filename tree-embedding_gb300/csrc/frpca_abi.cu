@@ -621,7 +621,9 @@ extern "C" tsvd_status tsvd_merge_svd(int32_t rows, int32_t cols, const double *
     TSVD_TRY(merge_matrix(W, m, rows, cols, dout, dsig, st));
     std::vector<float> hs(d);
     TSVD_CUDA(cudaMemcpyAsync(hs.data(), dsig, sizeof(float) * d, cudaMemcpyDeviceToHost, st));
+    TSVD_TRY(eig_sweeps_fetch(W, st));
     TSVD_CUDA(cudaStreamSynchronize(st));
+    TSVD_TRY(eig_check(W));
     for (int32_t j = 0; j < d; ++j) sigma[j] = hs[j];
     return fetch_columns(dout, d, nullptr, rows, stage, US, st);
   };

@@ -174,5 +174,6 @@ tsvd_status jacobi_eig_batched(double *const *g, int n, float *const *lambda,
                                int32_t *sweeps, int refine = 0,
                                const float *const *vinit = nullptr);
 size_t jacobi_work_bytes(int n, int nprob);
+constexpr int32_t kEigTimedOut = 1 << 20;  // *sweeps if a wait between CTAs ran out
 
 }  // namespace tsvd

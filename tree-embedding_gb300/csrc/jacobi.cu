@@ -28,8 +28,39 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
+__device__ __forceinline__ uint32_t remote_addr(uint32_t addr, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// Stores to a CTA of the cluster that count towards its barrier mbar.
+__device__ __forceinline__ void send_b32(uint32_t addr, float v, uint32_t mbar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
+      "r"(__float_as_uint(v)), "r"(mbar)
+      : "memory");
+}
+__device__ __forceinline__ void send_b64(uint32_t addr, uint64_t v, uint32_t mbar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+      "l"(v), "r"(mbar)
+      : "memory");
+}
+__device__ __forceinline__ bool try_wait(uint32_t mbar, uint32_t phase) {
+  uint32_t ok;
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(mbar), "r"(phase)
+      : "memory");
+  return ok != 0;
+}
+
 // ------------------------------------------------------------------ Jacobi
 constexpr int JAC_THREADS = 1024;
+constexpr int kJacWaits = 1 << 22;  // polls of a barrier before a cluster gives up
 constexpr int JAC_MAX_SWEEPS = 30;
 constexpr int kJacMaxCluster = 8;  // CTAs per eigenproblem (portable cluster size)
 constexpr int kJacRotBase = 512;   // first thread computing rotations (P <= 128 of them)
@@ -50,8 +81,8 @@ struct JacobiArgs {
 // Shared-memory layout of one CTA of jacobi_kernel (C CTAs per problem).
 struct JacobiSmem {
   int n, np, P, L, nbuf;
-  size_t off_dbase, off_lam, off_rows, off_pc, off_ps, off_pt, off_diag, off_coup, off_top,
-      off_bot, off_flag, bytes;
+  size_t off_dbase, off_lam, off_rows, off_cs, off_pt, off_diag, off_coup, off_top,
+      off_bot, off_slot, off_flag, off_mbar, bytes;
   __host__ __device__ JacobiSmem(int n_, int C) {
     n = n_;
     np = n + (n & 1);
@@ -62,14 +93,17 @@ struct JacobiSmem {
     off_dbase = o; o += (size_t)np * sizeof(double);
     off_lam = o; o += (size_t)np * sizeof(double);
     off_rows = o; o += (size_t)nbuf * np * sizeof(float);
-    off_pc = o; o += (size_t)P * sizeof(float);
-    off_ps = o; o += (size_t)P * sizeof(float);
+    off_cs = o; o += (size_t)P * sizeof(float2);
     off_pt = o; o += (size_t)P * sizeof(float);
     off_diag = o; o += (size_t)2 * np * sizeof(float);  // [parity][player]
     off_coup = o; o += (size_t)2 * P * sizeof(float);   // [parity][slot]
     off_top = o; o += (size_t)2 * L * sizeof(int);      // two map pairs (renamed each round)
     off_bot = o; o += (size_t)2 * L * sizeof(int);
-    off_flag = o; o += (size_t)(JAC_MAX_SWEEPS + 1) * sizeof(int);
+    o = (o + 7) & ~(size_t)7;
+    off_slot = o; o += (size_t)2 * L * sizeof(int2);    // [parity][slot]
+    off_flag = o; o += (size_t)(JAC_MAX_SWEEPS + 2) * sizeof(int);
+    o = (o + 7) & ~(size_t)7;
+    off_mbar = o; o += 2 * sizeof(uint64_t);  // [parity]
     bytes = (o + 15) & ~(size_t)15;
   }
 };
@@ -85,13 +119,16 @@ struct JacobiSmem {
 // different CTAs hold stay equal); then the schedule advances: each CTA
 // passes one row to each neighbour (into the neighbour's mailbox, in
 // distributed shared memory) and broadcasts, for every row it holds, the
-// diagonal entry and the coupling to the row's next partner; after the one
-// cluster barrier of the round, each CTA renames its rows (circle_arrivals,
-// circle_next) and computes all rotations of the next round itself, from the
-// same values in the same order, so every CTA has the same rotations without
-// a second exchange. Mailboxes and broadcast values alternate between two
-// buffers by round parity, so a fast CTA never overwrites what a slow one
-// has yet to read.
+// diagonal entry and the coupling to the row's next partner. These are stores that
+// count their bytes on a barrier in the receiver (st.async, mbarrier): a CTA goes on
+// when its round's bytes have come, one trip, where stores and a cluster barrier
+// after them take two. Meanwhile it renames its rows (circle_arrivals, circle_next);
+// then it computes all rotations of the next round itself, from the same values in
+// the same order, so every CTA has the same rotations without a second exchange.
+// Mailboxes, broadcast values and barriers alternate between two by round parity:
+// nobody sends for round g + 2 before it has what all others send in g + 1, and so
+// nothing is overwritten that is yet to be read. A wait that runs out (kJacWaits)
+// makes the CTA leave at the sweep's end, and the solve an error.
 //
 // Rotate when the pair is coupled: relative to the pair (Demmel-Veselic) and
 // above an absolute floor. The first pass only resolves the couplings above
@@ -107,14 +144,14 @@ struct JacobiSmem {
 // sits above the fp32 rounding its own rotations leave, so the tiny
 // eigenvalues' pairs cannot cycle.
 //
-// A round is a chain of latencies (update, barrier, send, cluster barrier,
-// rotations, barrier: 1.1 us at n = 256), so what a thread can know before the
-// loop or between the two halves of the cluster barrier is taken off the chain:
-// the divisions by P and C (a third of a round together with the renaming of the
-// rows by all 1024 threads), the row names, the angle beside its test; the first
-// pass does no fp64 arithmetic. The rotations and their order are those of the
-// plain loop. First pass, refinement and replay together, measured: n = 256
-// 8.55 -> 6.40 ms, 133 3.89 -> 2.69, 69 1.41 -> 0.97.
+// A round is a chain (clocks at n = 256, one problem: update 1800, which 32 warps'
+// issue bounds, sends and the wait for the others 1800, rotations 800), so what can
+// be known before the loop or while the data travel is taken off it: the divisions by
+// P and C, the row names and where each slot's rows begin, the players (one step on
+// the circle a round), the angle beside its test; the first pass does no fp64
+// arithmetic. The rotations and their order are those of the plain loop. First
+// pass, refinement and replay together, measured: n = 256 8.55 -> 5.2 ms, 133 3.89 ->
+// 2.24, 69 1.41 -> 0.79 (16 CTAs at n = 256: 5.5).
 __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
@@ -125,8 +162,7 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
   double *dbase = reinterpret_cast<double *>(jsm + lay.off_dbase);
   double *lam_all = reinterpret_cast<double *>(jsm + lay.off_lam);
   float *rows = reinterpret_cast<float *>(jsm + lay.off_rows);
-  float *pc = reinterpret_cast<float *>(jsm + lay.off_pc);
-  float *ps = reinterpret_cast<float *>(jsm + lay.off_ps);
+  float2 *rot = reinterpret_cast<float2 *>(jsm + lay.off_cs);  // cosine, sine of each slot
   float *pt = reinterpret_cast<float *>(jsm + lay.off_pt);
   float *diag = reinterpret_cast<float *>(jsm + lay.off_diag);  // [2][np]
   float *coup = reinterpret_cast<float *>(jsm + lay.off_coup);  // [2][P]
@@ -134,6 +170,8 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
   int *const bot_m = reinterpret_cast<int *>(jsm + lay.off_bot);
   int *flag = reinterpret_cast<int *>(jsm + lay.off_flag);  // [sweep]: some pair rotated
   int *top = top_m, *bot = bot_m;  // the current maps: slot s0+i -> row buffers
+  // where the rows of the slot's lower- and higher-numbered player begin
+  int2 *const slot_m = reinterpret_cast<int2 *>(jsm + lay.off_slot);
   const bool refine = a.refine != 0;
   const int prob = blockIdx.x / C;
   const int s0 = crank * L, nloc = min(P, s0 + L) - s0;  // >= 1 (host)
@@ -146,6 +184,7 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
   for (int i = threadIdx.x; i < nloc; i += blockDim.x) {
     top[i] = 2 * i;
     bot[i] = 2 * i + 1;
+    slot_m[i] = slot_m[L + i] = make_int2(2 * i * np, (2 * i + 1) * np);
   }
   for (int i = threadIdx.x; i < np; i += blockDim.x) {
     dbase[i] = (refine && i < n) ? Gin[(int64_t)i * n + i] : 0.0;
@@ -155,16 +194,23 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
     const int q = np - 1 - k;
     coup[k] = q < n ? (float)Gin[(int64_t)k * n + q] : 0.f;
   }
-  for (int i = threadIdx.x; i <= JAC_MAX_SWEEPS; i += blockDim.x) flag[i] = 0;
+  for (int i = threadIdx.x; i <= JAC_MAX_SWEEPS + 1; i += blockDim.x) flag[i] = 0;
+  volatile int *dead = flag + JAC_MAX_SWEEPS + 1;  // a wait ran out
+  const uint32_t sbase = smem_u32(jsm), mbar = sbase + (uint32_t)lay.off_mbar;
+  if (C > 1 && threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar + 8 * i) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   for (int idx = threadIdx.x; idx < 2 * nloc * np; idx += blockDim.x) {
     const int b = idx / np, col = idx % np, x = player_of(b);
     float v = 0.f;
     if (x < n && col < n && !(refine && x == col)) v = (float)Gin[(int64_t)x * n + col];
     rows[(size_t)b * np + col] = v;
   }
-  __syncthreads();
-  // Rotations of round t (of sweep `sw`, global round g) for every slot, from
-  // the broadcast values of parity `par`; threads < P.
+  if (C > 1) cluster.sync(); else __syncthreads();
+  // The rotation of slot k, players x and y (sweep `sw`, global round g), from the
+  // broadcast values of parity `par`.
   float dmax = 0.f;  // max|a_ii| at the start of the sweep (rotation warps)
   auto sweep_dmax = [&](int par) {
     float m = 0.f;
@@ -174,8 +220,7 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     return m;
   };
-  auto rotations = [&](int k, int t, int sw, int g, int par) {
-    const int x = circle_player(k, t, np), y = circle_player(np - 1 - k, t, np);
+  auto rotations = [&](int k, int x, int y, int sw, int g, int par) {
     const int p = min(x, y), q = max(x, y);
     float c = 1.f, s = 0.f, tt = 0.f;
     if (q < n) {
@@ -198,8 +243,7 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
         flag[sw] = 1;
       }
     }
-    pc[k] = c;
-    ps[k] = s;
+    rot[k] = make_float2(c, s);
     pt[k] = tt;
     if (k >= s0 && k < s0 + nloc) log[(int64_t)g * P + k] = make_float2(c, s);
   };
@@ -207,7 +251,7 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
   // 24-31, while warps 0-7 move rows, so the phases of a round overlap
   const int rt = (int)threadIdx.x - kJacRotBase, bt = (int)threadIdx.x - kJacSendBase;
   if (rt >= 0 && rt < ((P + 31) & ~31)) dmax = sweep_dmax(0);
-  if (rt >= 0 && rt < P) rotations(rt, 0, 0, 0, 0);
+  if (rt >= 0 && rt < P) rotations(rt, rt, np - 1 - rt, 0, 0, 0);
   __syncthreads();
   int sweeps_done = JAC_MAX_SWEEPS;
   // what a thread does every round, found once
@@ -216,6 +260,17 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
   const int bt_n = (JAC_THREADS - kJacSendBase) / C;
   const int bt_r = bt >= 0 ? bt % C : 0, bt_i = bt >= 0 ? bt / C : 2 * L;
   const bool updates = (int)threadIdx.x < cgroups * P;
+  // the players of column slot k2, or (rotation threads) of slot rt: one step on
+  // the circle a round
+  const int my = rt >= 0 && rt < P ? rt : k2;
+  int px = k2, py = np - 1 - k2, rx = my, ry = np - 1 - my;
+  auto step = [&](int x) { return x == 0 ? 0 : x == np - 1 ? 1 : x + 1; };
+  // shared memory of the CTAs this thread sends to: threads 0-127 the left
+  // neighbour's, 128-255 the right one's, from kJacSendBase on bt_r's
+  const int to = bt >= 0 ? bt_r : threadIdx.x < 128 ? max(crank - 1, 0) : min(crank + 1, C - 1);
+  const uint32_t rbase = remote_addr(sbase, to);
+  const uint32_t round_bytes =
+      4 * (np + P) + 4 * np * ((crank > 0 ? 1 : 0) + (crank < C - 1 ? 1 : 0));
   int t = 0, sw = 0;  // round of the sweep, sweep
   for (int g = 0;; ++g) {
     // every rotation applied to the owned rows, 2 x 2 block (owned slot k1,
@@ -223,29 +278,27 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
     // walks the owned slots (groups of P threads; the column pair's players
     // and rotation are loaded once)
     if (updates) {
-      const int x2 = circle_player(k2, t, np), y2 = circle_player(np - 1 - k2, t, np);
-      const int p2 = min(x2, y2), q2 = max(x2, y2);
-      const float c2 = pc[k2], s2v = ps[k2];
+      const int p2 = min(px, py), q2 = max(px, py);
+      const float2 r2 = rot[k2];
+      const float c2 = r2.x, s2v = r2.y;
+      const int2 *slot = slot_m + (g & 1) * L;
       for (int kl = kl0; kl < nloc; kl += cgroups) {
-        const int k1 = s0 + kl;
-        const float s1v = ps[k1];
+        const float2 r1 = rot[s0 + kl];
+        const float c1 = r1.x, s1v = r1.y;
         if (s1v == 0.f && s2v == 0.f) continue;
-        const int x1 = circle_player(k1, t, np), y1 = circle_player(np - 1 - k1, t, np);
-        const int p1 = min(x1, y1), q1 = max(x1, y1);
-        float *rp = rows + (x1 < y1 ? top[kl] : bot[kl]) * np;
-        float *rq = rows + (x1 < y1 ? bot[kl] : top[kl]) * np;
-        if (k2 == k1) {  // the rotation's own 2 x 2 block
-          const float t1 = pt[k1];
-          if (q1 < n && t1 != 0.f) {
-            const float apq = rp[q1];
-            rp[p1] -= t1 * apq;
-            rq[q1] += t1 * apq;
-            rp[q1] = 0.f;
-            rq[p1] = 0.f;
+        const int2 at = slot[kl];
+        float *rp = rows + at.x, *rq = rows + at.y;
+        if (k2 == s0 + kl) {  // the rotation's own 2 x 2 block
+          const float t1 = pt[k2];
+          if (q2 < n && t1 != 0.f) {
+            const float apq = rp[q2];
+            rp[p2] -= t1 * apq;
+            rq[q2] += t1 * apq;
+            rp[q2] = 0.f;
+            rq[p2] = 0.f;
           }
           continue;
         }
-        const float c1 = pc[k1];
         const float cc = __fmul_rn(c1, c2), cs = __fmul_rn(c1, s2v), sc = __fmul_rn(s1v, c2),
                     ss = __fmul_rn(s1v, s2v);
         const float b00 = rp[p2], b01 = rp[q2], b10 = rq[p2], b11 = rq[q2];
@@ -264,17 +317,22 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
     __syncthreads();
     // the next round: position j -> j - 1 (j >= 2), 1 -> np - 1, 0 stays
     const int g1 = g + 1, t1 = t + 1 == np - 1 ? 0 : t + 1, sw1 = t1 ? sw : sw + 1, par = g1 & 1;
-    float *mbox = rows + (size_t)(2 * L + 2 * par) * np;  // [from left, from right]
-    if (P >= 2) {  // hand-over: first owned top row left, last owned bottom row right
-      if (crank > 0) {
-        const float *src = rows + (size_t)top[0] * np;
-        float *dst = cluster.map_shared_rank(mbox, crank - 1) + np;
-        for (int i = threadIdx.x; i < np; i += blockDim.x) dst[i] = src[i];
-      }
-      if (crank < C - 1) {
-        const float *src = rows + (size_t)bot[nloc - 1] * np;
-        float *dst = cluster.map_shared_rank(mbox, crank + 1);
-        for (int i = threadIdx.x; i < np; i += blockDim.x) dst[i] = src[i];
+    const uint32_t bar = rbase + (uint32_t)lay.off_mbar + 8 * par;
+    if (C > 1) {
+      if (threadIdx.x == kJacRotBase - 32)  // the round's data, from every CTA
+        asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(
+                         mbar + 8 * par),
+                     "r"(round_bytes)
+                     : "memory");
+      // hand-over: first owned top row left, last owned bottom row right
+      if (threadIdx.x < 256) {
+        const int j = threadIdx.x & 127, left = threadIdx.x < 128;
+        const uint64_t *src =
+            reinterpret_cast<const uint64_t *>(rows + (size_t)(left ? top[0] : bot[nloc - 1]) * np);
+        const uint32_t dst = rbase + (uint32_t)lay.off_rows +
+                             4 * (uint32_t)((2 * L + 2 * par + left) * np) + 8 * j;
+        if (left ? crank > 0 : crank < C - 1)
+          if (j < np / 2) send_b64(dst, src[j], bar);
       }
     }
     // each held row's diagonal, and its coupling to its next partner (sent by
@@ -285,44 +343,80 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
       const float *row = rows + (size_t)((i & 1) ? bot[i / 2] : top[i / 2]) * np;
       const int pos1 = pos == 0 ? 0 : (pos == 1 ? np - 1 : pos - 1);
       const int k1 = min(pos1, np - 1 - pos1), y = circle_player(np - 1 - pos1, t1, np);
-      cluster.map_shared_rank(diag, bt_r)[par * np + x] = row[x];
-      if (x < y) cluster.map_shared_rank(coup, bt_r)[par * P + k1] = y < n ? row[y] : 0.f;
+      const float dx = row[x], cx = x < y && y < n ? row[y] : 0.f;
+      if (C > 1) {
+        send_b32(rbase + (uint32_t)lay.off_diag + 4 * (par * np + x), dx, bar);
+        if (x < y) send_b32(rbase + (uint32_t)lay.off_coup + 4 * (par * P + k1), cx, bar);
+      } else {
+        diag[par * np + x] = dx;
+        if (x < y) coup[par * P + k1] = cx;
+      }
     }
-    // the row names of the next round are worked out between the two halves of
-    // the barrier (only this CTA's maps are involved)
-    if (C > 1) cluster.barrier_arrive();
+    // the row names of the next round, while the data travel (only this CTA's maps
+    // are involved)
     int dl = -1, dr = -1;
     int *ntop = top == top_m ? top_m + L : top_m, *nbot = bot == bot_m ? bot_m + L : bot_m;
     if (P >= 2 && (int)threadIdx.x < 256) {
       circle_arrivals(top, bot, s0, nloc, P, &dl, &dr);
       for (int i = threadIdx.x; i < nloc; i += 256)
-        circle_next(top, bot, s0, nloc, P, i, dl, dr, &ntop[i], &nbot[i]);
+      {
+        int nt, nb;
+        circle_next(top, bot, s0, nloc, P, i, dl, dr, &nt, &nb);
+        ntop[i] = nt;
+        nbot[i] = nb;
+        const bool up = circle_player(s0 + i, t1, np) < circle_player(np - 1 - s0 - i, t1, np);
+        slot_m[par * L + i] = up ? make_int2(nt * np, nb * np) : make_int2(nb * np, nt * np);
+      }
     }
-    if (C > 1) cluster.barrier_wait(); else __syncthreads();  // a one-CTA barrier is 8x cheaper
-    if (P >= 2) {  // arrived rows take the freed buffers
-      for (int i = threadIdx.x; i < np && i < 256; i += 256) {
+    px = step(px);
+    py = step(py);
+    rx = step(rx);
+    ry = step(ry);
+    if (C > 1) {
+      if (threadIdx.x < 256 || (rt >= 0 && rt < ((P + 31) & ~31))) {
+        const uint32_t phase = ((uint32_t)(g1 - 1) >> 1) & 1;
+        int polls = 0;
+        while (!try_wait(mbar + 8 * par, phase))
+          if (*dead || ++polls > kJacWaits) {
+            *dead = 1;
+            break;
+          }
+      }
+      // the rows sent are overwritten next: their readers, warps 0-7 and 24-31, are done
+      if (threadIdx.x < 256)
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+      else if (bt >= 0)
+        asm volatile("bar.arrive 1, 512;" ::: "memory");
+      if (P >= 2 && (int)threadIdx.x < np) {  // arrived rows take the freed buffers
+        const float *mbox = rows + (size_t)(2 * L + 2 * par) * np;  // [from left, from right]
+        const int i = threadIdx.x;
         if (dl >= 0) rows[(size_t)dl * np + i] = mbox[i];
         if (dr >= 0) rows[(size_t)dr * np + i] = mbox[np + i];
       }
+    } else {
+      __syncthreads();
+    }
+    if (P >= 2) {
       top = ntop;
       bot = nbot;
     }
     if (t1 == 0) {  // sweep boundary: stop after a sweep without rotations
       __syncthreads();
-      if (!flag[sw1 - 1] || sw1 == JAC_MAX_SWEEPS) {  // the same in every CTA
+      // (the same in every CTA, but for a wait that ran out)
+      if (!flag[sw1 - 1] || sw1 == JAC_MAX_SWEEPS || *dead) {
         sweeps_done = sw1;
         break;
       }
       if (rt >= 0 && rt < ((P + 31) & ~31)) dmax = sweep_dmax(par);
     }
-    if (rt >= 0 && rt < P) rotations(rt, t1, sw1, g1, par);
+    if (rt >= 0 && rt < P) rotations(rt, rx, ry, sw1, g1, par);
     __syncthreads();
     t = t1;
     sw = sw1;
   }
   if (crank == 0 && threadIdx.x == 0) {
     a.sweeps[prob] = sweeps_done;
-    atomicMax(a.most_sweeps, sweeps_done);
+    atomicMax(a.most_sweeps, *dead ? kEigTimedOut : sweeps_done);
   }
   // eigenvalues to every CTA of the cluster, then each ranks its own players
   for (int i = threadIdx.x; i < 2 * nloc; i += blockDim.x) {
