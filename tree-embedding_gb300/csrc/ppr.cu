@@ -19,6 +19,19 @@
 // a non-zero degree (collect_kernel over the touched bitset).
 // The loop ends when a frontier is empty: every eligible residue <= rmax,
 // the same invariant the FIFO leaves behind.
+//
+// Within a round the items run side by side: one that is read late has already
+// received what the early ones scatter, and a vertex of more than kHeavy neighbours
+// scatters after all others. The order of the items, what scatters at once and the
+// pace of the launches decide which of the many valid end states a push reaches
+// (two runs of one push differ by 1e-3 to 2e-2 in the embedding's E E^T), so a change
+// to any of them moves every embedding, by more than a run does where it is
+// systematic: with vertices of more than 256 neighbours last in their round, the mean
+// of 14 runs moved 2 to 4 times as far as between two such means without a change. In a
+// small graph even where its arrays lie shows: 512 bytes more before them moved the mean
+// of the 4,000-vertex tenant (64 sources) by 1e-3, five times as far as nothing did, so
+// the device allocations below are counted too. What differs here by the size of the
+// graph (kLargePairs) was chosen so that neither the mean nor the spread moves.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -31,21 +44,8 @@ namespace tsvd {
 
 namespace {
 
+constexpr int kHeavy = 1024;  // neighbours per warp work unit for hub vertices
 constexpr unsigned kFull = 0xffffffffu;
-
-// Neighbours a warp takes in one piece; vertices with more are split into units for
-// push_heavy_kernel, by the items of the round. In a large round long pieces cost
-// nothing, as other warps have other items; each unit is a slot and a weight read
-// more, and what a hub scatters at once, before the vertices after it are read, they
-// push in the same round and not in one more. In a small round a piece is what the
-// round waits for: 1024 neighbours take one warp 30 us, 128 take 5, and the tail of
-// a push is some 50 such rounds. Push stage, ms, 128 up to 2^18 items and 1024 above
-// / these: 4,000 vertices 0.82 / 0.63, 100k 8.5 / 7.6, Wikipedia-like 87 / 82,
-// Patent-like 30.4 / 30.2 (4096 and more in the largest rounds 31.1 to 32.8, 16 in the
-// smallest 0.71). Rounds of up to 2^18 items cannot overflow the slots.
-__device__ __forceinline__ int32_t piece_for(int32_t nitems) {
-  return nitems < (1 << 12) ? 32 : nitems < (1 << 15) ? 128 : nitems < (1 << 18) ? 512 : 2048;
-}
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -85,6 +85,12 @@ __device__ __forceinline__ void flush_stats(const StatAcc &acc, unsigned long lo
 // collect_kernel. Each half-warp takes one neighbour per instruction, lane q
 // adding sources 4q..4q+3 as one float4 (RED.v4): two 256-byte runs per warp
 // instruction, half the L1 requests of one float2 per lane and neighbour.
+// TEST (large graphs): a touched bit is read first and set only where it is not. A mark
+// costs L2 a sector like each of the run's, of which the scatter is bound, and in a
+// dense round 28 of 29 change nothing. Steps, marks always set / tested: 150k vertices
+// of degree 29 128 -> 107 ms, 300k of degree 5 59 -> 53 ms, 100k undirected 21.3 -> 19.4
+// ms; in a graph of few pairs (4,000 vertices, 64 sources) 3.3 ms both ways.
+template <bool TEST>
 __device__ __forceinline__ void scatter_range(const PushArgs &a, const int32_t *nb, int32_t c,
                                               float2 w, int32_t j0, int32_t j1, int32_t mine) {
   const int lane = threadIdx.x & 31;
@@ -103,41 +109,37 @@ __device__ __forceinline__ void scatter_range(const PushArgs &a, const int32_t *
     // the touched bit of the neighbour this lane loaded, as it is now in L2
     const int64_t idx = (int64_t)c * a.n + mine;
     const uint32_t bit = 1u << (idx & 31);
-    const uint32_t seen = lane < jn ? __ldcg(a.tflag + (idx >> 5)) : bit;
+    const uint32_t seen = TEST && lane < jn ? __ldcg(a.tflag + (idx >> 5)) : 0u;
     for (int32_t t = 0; t < jn; t += 2) {
       const int32_t u = __shfl_sync(kFull, mine, (t + half) & 31);
       if (act && t + half < jn) atomicAdd(rc + (int64_t)u * (kChunk / 4), w4);
     }
-    // Each lane marks the neighbour it loaded, unless it is marked: a reduction
-    // costs L2 a sector like each of the run's, of which the scatter is bound,
-    // and in a dense round 28 of 29 marks change nothing.
-    if (!(seen & bit)) atomicOr(a.tflag + (idx >> 5), bit);
+    // each lane marks the neighbour it loaded: 32 independent reductions
+    if (TEST) {
+      if (lane < jn && !(seen & bit)) atomicOr(a.tflag + (idx >> 5), bit);
+    } else if (lane < jn) {
+      mark_pair(a.tflag, mine, c, a.n);
+    }
     mine = next;
   }
 }
 
-// One warp per item, a fixed share of the items each, on a grid of resident
-// blocks (5 a SM; the blocks of a second wave, as with 8 a SM, ran alone at the
-// end). What bounds a dense round is L2's rate of reducing 32-byte sectors:
-// 200-238 G/s here, and 205 G/s for whole random runs that all hit L2 (25.6 G
-// runs/s; half runs 52 G/s). Sharing the items out through a counter kept every
-// SM busy and was slower, its atomics queueing behind the reductions.
-__global__ void __launch_bounds__(256, 5) push_kernel(PushArgs a) {
+// One warp per item, a fixed share of the items each. What bounds a dense round is
+// L2's rate of reducing 32-byte sectors: 200-238 G/s here, and 205 G/s for whole random
+// runs that all hit L2 (25.6 G runs/s; half runs 52 G/s).
+template <bool TEST>
+__global__ void __launch_bounds__(256) push_kernel(PushArgs a) {
   const int lane = threadIdx.x & 31;
-  const int32_t gw = (int32_t)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-  const int32_t nw = (int32_t)(((int64_t)gridDim.x * blockDim.x) >> 5);
-  const int32_t nlight = a.front_count[0], nitems = nlight + a.front_count[kHighCount];
-  const int32_t piece = piece_for(nitems);
-  auto item = [&](int32_t i) {
-    return __ldg(i < nlight ? a.front + i : a.front + (a.cap - 1 - (i - nlight)));
-  };
-  if (gw == 0 && lane == 0) a.stats[kStatSlots * 4] = global_ns();
+  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int32_t nitems = *a.front_count;
+  if (TEST && gw == 0 && lane == 0) a.clock[0] = global_ns();
   StatAcc acc;
-  int2 it = gw < nitems ? item(gw) : make_int2(0, 0);
-  for (int32_t i = gw; i < nitems; i += nw) {
+  int2 it = gw < nitems ? __ldg(a.front + gw) : make_int2(0, 0);
+  for (int64_t i = gw; i < nitems; i += nw) {
     const int32_t v = it.x, c = it.y;
     // the warp's next item is loaded while this one is pushed
-    it = i + nw < nitems ? item(i + nw) : make_int2(0, 0);
+    it = i + nw < nitems ? __ldg(a.front + i + nw) : make_int2(0, 0);
     // Everything the item needs that does not depend on its residues is
     // requested at once: degree, row start, reserve line, first neighbour ids
     // (only this warp writes the reserve of (v, chunk c) in a round).
@@ -196,10 +198,10 @@ __global__ void __launch_bounds__(256, 5) push_kernel(PushArgs a) {
       acc.items += 1;
       acc.iedges += (unsigned long long)d;
     }
-    if (d > piece) {
+    if (d > kHeavy) {
       // Hub vertex: park the lane weights and split the neighbour list into
-      // piece-sized units processed by push_heavy_kernel.
-      const int32_t units = (d + piece - 1) / piece;
+      // kHeavy-sized units processed by push_heavy_kernel.
+      const int32_t units = (d + kHeavy - 1) / kHeavy;
       int32_t slot = 0, u0 = 0, ok = 0;
       if (lane == 0) {
         slot = atomicAdd(a.heavy_count, 1);
@@ -216,69 +218,147 @@ __global__ void __launch_bounds__(256, 5) push_kernel(PushArgs a) {
       }
       if (units_reserved)
         for (int32_t k = lane; k < units; k += 32)
-          a.units[u0 + k] = make_int2(ok ? slot : -1, k * piece);
+          a.units[u0 + k] = make_int2(ok ? slot : -1, k * kHeavy);
       if (ok) continue;
       // buffers full: process this hub inline
     }
-    scatter_range(a, nb, c, w, 0, d, mine0);
+    scatter_range<TEST>(a, nb, c, w, 0, d, mine0);
   }
   flush_stats(acc, a.stats);
 }
 
+template <bool TEST>
 __global__ void __launch_bounds__(256) push_heavy_kernel(PushArgs a) {
   const int lane = threadIdx.x & 31;
-  const int32_t gw = (int32_t)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-  const int32_t nw = (int32_t)(((int64_t)gridDim.x * blockDim.x) >> 5);
+  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int32_t nunits = min(*a.unit_count, a.unit_cap);
-  const int32_t piece = piece_for(a.front_count[0] + a.front_count[kHighCount]);
-  for (int32_t i = gw; i < nunits; i += nw) {
-    const int2 u = a.units[i];
+  for (int64_t i = gw; i < nunits; i += nw) {
+    int2 u = a.units[i];
     if (u.x < 0) continue;
-    const int2 it = a.heavy_item[u.x];
+    int2 it = a.heavy_item[u.x];
     const float2 w = reinterpret_cast<const float2 *>(a.heavy_w)[(int64_t)u.x * 32 + lane];
     const int32_t d = a.deg[it.x];
     const int32_t *nb = a.nbr + a.off[it.x];
-    const int32_t j1 = min(d, u.y + piece);
+    const int32_t j1 = min(d, u.y + kHeavy);
     const int32_t mine0 = lane < j1 - u.y ? __ldg(nb + u.y + lane) : 0;
-    scatter_range(a, nb, it.y, w, u.y, j1, mine0);
+    scatter_range<TEST>(a, nb, it.y, w, u.y, j1, mine0);
   }
 }
 
 // Scan the touched bitset; for each touched (u, chunk) with some residue
 // above theta and deg(u) > 0, append it to the next frontier. Clears the bits.
-// A warp lists the set bits of its words (up to eight) in shared memory and
-// takes them eight at a time: lane group g (4 lanes) reads pair g's 256-byte
-// residue run as sixteen float4 (four per lane), so eight runs are in flight
-// per warp. Padding sources (s >= |S|) hold zero residue. A dense bitset is
-// read at the bandwidth of L2; a sparse one waits for latencies, about two per
-// eight pairs, which is why the pairs of all eight words are taken together
-// (word by word, two bits a word cost as much as eight).
+// A warp takes the set bits of a word eight at a time: lane group g (4 lanes)
+// reads pair g's 256-byte residue run as sixteen float4 (four per lane), so
+// eight runs are in flight per warp. Padding sources (s >= |S|) hold zero
+// residue.
 __global__ void __launch_bounds__(256) collect_kernel(CollectArgs a) {
-  __shared__ int2 buf[2048];  // light items from the start, the others from the end
+  __shared__ int2 buf[2048];
+  __shared__ int32_t nbuf, gbase;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int grp = lane >> 2, gl = lane & 3;
+  const int64_t words_per_iter = 64;  // 8 warps x 8 words
+  for (int64_t w0 = (int64_t)blockIdx.x * words_per_iter; w0 < a.nwords;
+       w0 += (int64_t)gridDim.x * words_per_iter) {
+    if (threadIdx.x == 0) nbuf = 0;
+    // the warp's eight words in one load (lanes 0-7): in the late rounds of a
+    // push almost every word is zero, and eight dependent loads per warp made
+    // the scan of the bitset cost 0.14 ms a round
+    const int64_t wbase = w0 + warp * 8;
+    const uint32_t wv = (lane < 8 && wbase + lane < a.nwords) ? __ldcg(a.tflag + wbase + lane) : 0u;
+    __syncthreads();
+    for (int k = 0; k < 8; ++k) {
+      const int64_t wi = wbase + k;
+      if (wi >= a.nwords) break;
+      uint32_t bits = __shfl_sync(kFull, wv, k);
+      if (!bits) continue;
+      if (lane == 0) a.tflag[wi] = 0;
+      while (bits) {
+        // the next (up to) eight set bits, one per lane group
+        uint32_t rest = bits;
+        int mybit = -1;
+        for (int g = 0; g < 8 && rest; ++g) {
+          const int bpos = __ffs(rest) - 1;
+          rest &= rest - 1;
+          if (g == grp) mybit = bpos;
+        }
+        bits = rest;
+        int32_t u = 0, c = 0, du = 0;
+        bool live = mybit >= 0;
+        if (live) {
+          const int64_t idx = wi * 32 + mybit;
+          u = (int32_t)(idx % a.n);
+          c = (int32_t)(idx / a.n);
+          du = a.deg[u];
+          live = du != 0;
+        }
+        const float th = (a.hub_deg > 0 && du < a.hub_deg) ? a.rmax_f : a.theta_f;
+        float m = 0.f;
+        if (live) {
+          const float4 *line =
+              reinterpret_cast<const float4 *>(a.r + ppr_cell(u, c * kChunk, a.n));
+          const float4 x0 = __ldcg(line + gl), x1 = __ldcg(line + gl + 4);
+          const float4 x2 = __ldcg(line + gl + 8), x3 = __ldcg(line + gl + 12);
+          const float m0 = fmaxf(fmaxf(fmaxf(x0.x, x0.y), fmaxf(x0.z, x0.w)),
+                                 fmaxf(fmaxf(x1.x, x1.y), fmaxf(x1.z, x1.w)));
+          const float m1 = fmaxf(fmaxf(fmaxf(x2.x, x2.y), fmaxf(x2.z, x2.w)),
+                                 fmaxf(fmaxf(x3.x, x3.y), fmaxf(x3.z, x3.w)));
+          m = fmaxf(m0, m1);
+        }
+        const unsigned above = __ballot_sync(kFull, live && m > th);
+        const unsigned parked =
+            __ballot_sync(kFull, live && th > a.rmax_f && m > a.rmax_f) & ~above;
+        const unsigned gmask = 0xFu << (grp * 4);
+        if (gl == 0 && live) {
+          if (above & gmask) buf[atomicAdd(&nbuf, 1)] = make_int2(u, c);
+          else if (parked & gmask) mark_pair(a.pend, u, c, a.n);  // for a lower level
+        }
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) gbase = nbuf ? atomicAdd(a.next_count, nbuf) : 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < nbuf; i += blockDim.x) {
+      const int64_t dst = (int64_t)gbase + i;
+      if (dst < a.cap) a.next[dst] = buf[i];
+      else atomicExch(a.overflow, 1);
+    }
+    __syncthreads();
+  }
+}
+
+// The same for large graphs. A warp lists the set bits of its eight words in shared
+// memory and takes them sixteen at a time, in two sets of eight. A dense bitset is read
+// at the bandwidth of L2; a sparse one waits for latencies, about two per sixteen
+// pairs, where word by word two bits a word cost as much as eight. Steps, word by word
+// / this: 150k vertices of degree 29 109 -> 106 ms, 100k undirected 19.4 -> 18.3.
+__global__ void __launch_bounds__(256) collect_large_kernel(CollectArgs a) {
+  __shared__ int2 buf[2048];
   __shared__ uint8_t list[8][256];  // bit within the warp's words
-  __shared__ int32_t nbuf[2], gbase[2];
+  __shared__ int32_t nbuf, gbase;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int grp = lane >> 2, gl = lane & 3;
   const unsigned below = (1u << lane) - 1u;
-  const int64_t words_per_iter = 8 * a.words;
-  if (a.spent && blockIdx.x == 0 && threadIdx.x < 8) {
-    // the round's counters start at zero again (its scatter kernels are done)
+  const int64_t words_per_iter = 64;  // 8 warps x 8 words
+  // In a round one block more is launched: its scatter kernels are done, and their
+  // counters start at zero again.
+  const int nblocks = (int)gridDim.x - (a.spent ? 1 : 0);
+  if ((int)blockIdx.x == nblocks) {
+    if (threadIdx.x < 2) a.round[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
-      a.spent[0] = a.spent[kHighCount] = 0;
+      *a.spent = 0;
       a.clock[1] += global_ns() - a.clock[0];
     }
-    if (threadIdx.x == 2 || threadIdx.x == 3) a.round[threadIdx.x - 2] = 0;
+    return;
   }
   for (int64_t w0 = (int64_t)blockIdx.x * words_per_iter; w0 < a.nwords;
-       w0 += (int64_t)gridDim.x * words_per_iter) {
-    if (threadIdx.x < 2) nbuf[threadIdx.x] = 0;
-    // The warp's words in one load: in the late rounds of a push almost every
-    // word is zero. A small bitset is spread over the warps there are, down to
-    // a word each: with eight words a warp the 125 words of a 4000-vertex graph
-    // kept two blocks busy for 37 us.
-    const int64_t wbase = w0 + warp * a.words;
+       w0 += (int64_t)nblocks * words_per_iter) {
+    if (threadIdx.x == 0) nbuf = 0;
+    // the warp's words in one load: in the late rounds of a push almost every
+    // word is zero
+    const int64_t wbase = w0 + warp * 8;
     const int wk = lane >> 2;  // this lane's word and byte
-    const bool mine = wk < a.words && wbase + wk < a.nwords;
+    const bool mine = wbase + wk < a.nwords;
     const uint32_t word = mine ? __ldcg(a.tflag + wbase + wk) : 0u;
     if (word && gl == 0) a.tflag[wbase + wk] = 0;
     uint32_t byte = (word >> (8 * gl)) & 0xffu;
@@ -333,30 +413,22 @@ __global__ void __launch_bounds__(256) collect_kernel(CollectArgs a) {
             __ballot_sync(kFull, live && th > a.rmax_f && m > a.rmax_f) & ~above;
         const unsigned gmask = 0xFu << (grp * 4);
         const bool lead = gl == 0 && live, take = lead && (above & gmask);
-        const bool high = du[k] > a.light;
-        // one shared atomic per class
-        const unsigned mlow = __ballot_sync(kFull, take && !high),
-                       mhigh = __ballot_sync(kFull, take && high);
-        if (mlow | mhigh) {
+        const unsigned taken = __ballot_sync(kFull, take);
+        if (taken) {
           int slot = 0;
-          if (lane < 2) slot = atomicAdd(&nbuf[lane], __popc(lane ? mhigh : mlow));
-          const int low_at = __shfl_sync(kFull, slot, 0), high_at = __shfl_sync(kFull, slot, 1);
-          if (take)
-            buf[high ? 2047 - (high_at + __popc(mhigh & below)) : low_at + __popc(mlow & below)] =
-                make_int2(u[k], c[k]);
+          if (lane == 0) slot = atomicAdd(&nbuf, __popc(taken));
+          slot = __shfl_sync(kFull, slot, 0);
+          if (take) buf[slot + __popc(taken & below)] = make_int2(u[k], c[k]);
         }
         if (lead && !take && (parked & gmask)) mark_pair(a.pend, u[k], c[k], a.n);  // a lower level
       }
     }
     __syncthreads();
-    if (threadIdx.x < 2)
-      gbase[threadIdx.x] = nbuf[threadIdx.x] ? atomicAdd(a.next_count + kHighCount * threadIdx.x,
-                                                         nbuf[threadIdx.x]) : 0;
+    if (threadIdx.x == 0) gbase = nbuf ? atomicAdd(a.next_count, nbuf) : 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < nbuf[0] + nbuf[1]; i += blockDim.x) {
-      const int high = i >= nbuf[0], k = high ? i - nbuf[0] : i;
-      const int64_t dst = (int64_t)gbase[high] + k;
-      if (dst < a.cap) a.next[high ? a.cap - 1 - dst : dst] = buf[high ? 2047 - k : k];
+    for (int i = threadIdx.x; i < nbuf; i += blockDim.x) {
+      const int64_t dst = (int64_t)gbase + i;
+      if (dst < a.cap) a.next[dst] = buf[i];
       else atomicExch(a.overflow, 1);
     }
     __syncthreads();
@@ -459,10 +531,7 @@ __global__ void init_sources_kernel(const int32_t *__restrict__ sources, int32_t
     r[ppr_cell(v, k, n)] = 1.0f;
     front[k] = make_int2(v, k / kChunk);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    count[0] = nsrc;
-    count[kHighCount] = 0;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *count = nsrc;
 }
 
 // Zero fill with 16-byte stores (also for p in mapped host memory).
@@ -488,25 +557,22 @@ float largest_float_not_above(double x) {
 
 }  // namespace
 
-// Blocks of 256 threads the kernel keeps resident on the whole GPU.
-static int resident_blocks(const void *fn) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0) != cudaSuccess) {
-    cudaGetLastError();
-    per_sm = 4;
-  }
-  return sm_count() * std::max(per_sm, 1);
+// Blocks that cover the touched bitset, 64 words each.
+static int collect_grid(const PprState &P) {
+  return grid_for(ceil_div(P.nwords, 64) * 256, 256, 8);
 }
 
-static int32_t light_degree(const PprState &P) {
-  return P.cap < kLightPairs ? INT32_MAX : kLightDegree;
-}
+static bool is_large(const PprState &P) { return P.cap >= kLargePairs; }
 
-// collect_kernel's grid and words per warp for a bitset of nwords words.
-static int collect_grid(int64_t nwords, int *words) {
-  static const int resident = resident_blocks((const void *)collect_kernel);
-  *words = (int)std::max<int64_t>(1, std::min<int64_t>(8, ceil_div(nwords, (int64_t)resident * 8)));
-  return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(nwords, 8ll * *words), resident));
+// Outside a round: nothing but the frontier.
+static tsvd_status collect_launch(const PprState &P, CollectArgs ca, cudaStream_t st) {
+  ca.spent = nullptr;
+  if (is_large(P))
+    collect_large_kernel<<<collect_grid(P), 256, 0, st>>>(ca);
+  else
+    collect_kernel<<<collect_grid(P), 256, 0, st>>>(ca);
+  TSVD_LAUNCH_CHECK();
+  return TSVD_OK;
 }
 
 tsvd_status ppr_alloc(PprState &P, int32_t n, int32_t nsrc, int32_t sp, bool host_reserve) {
@@ -548,9 +614,9 @@ tsvd_status ppr_alloc(PprState &P, int32_t n, int32_t nsrc, int32_t sp, bool hos
   TSVD_CUDA(cudaMalloc(&P.heavy_item, (size_t)P.heavy_cap * sizeof(int2)));
   TSVD_CUDA(cudaMalloc(&P.units, (size_t)P.unit_cap * sizeof(int2)));
   TSVD_CUDA(cudaMalloc(&P.upd, (size_t)n * sizeof(int32_t)));
-  TSVD_CUDA(cudaMalloc(&P.counters, kCounters * sizeof(int32_t)));
-  TSVD_CUDA(cudaMemset(P.counters, 0, kCounters * sizeof(int32_t)));
-  TSVD_CUDA(cudaMalloc(&P.stats, (kStatSlots * 4 + 2) * sizeof(unsigned long long)));
+  TSVD_CUDA(cudaMalloc(&P.counters, 2 * kCounters * sizeof(int32_t)));
+  TSVD_CUDA(cudaMemset(P.counters, 0, 2 * kCounters * sizeof(int32_t)));
+  TSVD_CUDA(cudaMalloc(&P.stats, kStatSlots * 4 * sizeof(unsigned long long)));
   TSVD_CUDA(cudaMallocHost(&P.host_counters, 2 * kCounters * sizeof(int32_t)));
   for (auto &e : P.kev) TSVD_CUDA(cudaEventCreate(&e));
   return TSVD_OK;
@@ -576,8 +642,8 @@ void ppr_free(PprState &P) {
 }
 
 // counters: [0],[1] frontier counts, [2] heavy count, [3] unit count,
-// [4] overflow flag, [5] number of updated vertices, [8],[9] frontier counts of
-// the items that are not light.
+// [4] overflow flag, [5] number of updated vertices; large graphs: [8..9] start of the
+// round and [10..11] time of the scatter kernels so far, in ns.
 tsvd_status ppr_refresh(PprState &P, const Adjacency &A, const int32_t *sources_dev,
                         bool from_scratch, const PprParams &prm, uint8_t *vmark,
                         cudaStream_t st) {
@@ -587,6 +653,7 @@ tsvd_status ppr_refresh(PprState &P, const Adjacency &A, const int32_t *sources_
     TSVD_TRY(zero_floats(P.p, (size_t)P.n * P.sp, st));
     TSVD_CUDA(cudaMemsetAsync(P.tflag, 0, P.nwords * sizeof(uint32_t), st));
     TSVD_CUDA(cudaMemsetAsync(P.pend, 0, P.nwords * sizeof(uint32_t), st));
+    P.cur = 0;
     init_sources_kernel<<<grid_for(P.nsrc, 256), 256, 0, st>>>(sources_dev, P.nsrc, P.r, P.n,
                                                                   P.front[0], P.counters + 0);
     TSVD_LAUNCH_CHECK();
@@ -604,34 +671,32 @@ tsvd_status ppr_refresh(PprState &P, const Adjacency &A, const int32_t *sources_
   refresh_kernel<<<grid_for((A.n + 31) / 32 * (int64_t)P.chunks * 32, 256, 16), 256, 0, st>>>(ra);
   TSVD_LAUNCH_CHECK();
   // seed the frontier from the touched (vertex, chunk) pairs
-  TSVD_CUDA(cudaMemsetAsync(P.counters, 0, kCounters * sizeof(int32_t), st));
+  P.cur = 0;
+  TSVD_CUDA(cudaMemsetAsync(P.counters + 0, 0, sizeof(int32_t), st));
   CollectArgs ca;
   ca.tflag = P.tflag; ca.nwords = P.nwords; ca.n = P.n; ca.chunks = P.chunks; ca.nsrc = P.nsrc;
   ca.sp = P.sp; ca.r = P.r; ca.deg = A.deg; ca.rmax_f = largest_float_not_above(prm.rmax);
   ca.theta_f = ca.rmax_f; ca.hub_deg = 0; ca.pend = P.pend;
   ca.next = P.front[0]; ca.next_count = P.counters + 0; ca.cap = P.cap;
   ca.overflow = P.counters + 4;
-  ca.spent = nullptr;
-  ca.light = light_degree(P);
-  const int gcol = collect_grid(P.nwords, &ca.words);
-  collect_kernel<<<gcol, 256, 0, st>>>(ca);
-  TSVD_LAUNCH_CHECK();
+  TSVD_TRY(collect_launch(P, ca, st));
   P.seeded = true;
   return TSVD_OK;
 }
 
 namespace {
 
-// One push (one PPR state), advanced kRounds rounds at a time.
+// One push (one PPR state), advanced a few rounds at a time.
 struct PushJob {
   PprState *P = nullptr;
   cudaStream_t st = nullptr;
   PushArgs pa;  // zeroed by job_begin, padding too: compared as bytes
   CollectArgs ca;
-  int gpush = 0, gheavy = 0, gcol = 0;
+  int gpush = 0, gcol = 0;
   int level = 0;
   bool done = false;
   int64_t rounds = 0;
+  double kernel_ms = 0;
 };
 
 tsvd_status job_begin(PushJob &J, PprState &P, const Adjacency &A, const PprParams &prm,
@@ -639,11 +704,8 @@ tsvd_status job_begin(PushJob &J, PprState &P, const Adjacency &A, const PprPara
   if (!P.seeded) return fail(TSVD_ERR_STATE, "push before refresh");
   J.P = &P;
   J.st = st;
-  TSVD_CUDA(cudaMemsetAsync(P.stats, 0, (kStatSlots * 4 + 2) * sizeof(unsigned long long), st));
-  // every counter but the frontier's (the refresh leaves it in counters[0] and
-  // counters[kHighCount])
-  TSVD_CUDA(cudaMemsetAsync(P.counters + 1, 0, 7 * sizeof(int32_t), st));
-  TSVD_CUDA(cudaMemsetAsync(P.counters + 9, 0, sizeof(int32_t), st));
+  TSVD_CUDA(cudaMemsetAsync(P.stats, 0, kStatSlots * 4 * sizeof(unsigned long long), st));
+  TSVD_CUDA(cudaMemsetAsync(P.counters + 4, 0, sizeof(int32_t), st));
   std::memset(&J.pa, 0, sizeof J.pa);
   std::memset(&J.ca, 0, sizeof J.ca);
   const float rmax_f = largest_float_not_above(prm.rmax);
@@ -654,7 +716,6 @@ tsvd_status job_begin(PushJob &J, PprState &P, const Adjacency &A, const PprPara
   pa.rmax_f = rmax_f; pa.undirected = prm.undirected; pa.vmark = vmark;
   pa.hub_deg = prm.hub_degree;
   pa.co_f = prm.cofrac >= 1.0 ? rmax_f : (float)(prm.rmax * std::max(prm.cofrac, 0.0));
-  pa.cap = P.cap;
   pa.heavy_w = P.heavy_w; pa.heavy_item = P.heavy_item;
   pa.heavy_count = P.counters + 2; pa.heavy_cap = P.heavy_cap;
   pa.units = P.units; pa.unit_count = P.counters + 3; pa.unit_cap = P.unit_cap;
@@ -664,16 +725,19 @@ tsvd_status job_begin(PushJob &J, PprState &P, const Adjacency &A, const PprPara
   ca.nsrc = P.nsrc; ca.sp = P.sp; ca.r = P.r; ca.deg = A.deg; ca.rmax_f = rmax_f;
   ca.cap = P.cap; ca.overflow = P.counters + 4;
   ca.hub_deg = prm.hub_degree;
-  ca.light = light_degree(P);
-  ca.round = P.counters + 2; ca.clock = P.stats + kStatSlots * 4;
-  static const int push_resident = resident_blocks((const void *)push_kernel);
-  static const int heavy_resident = resident_blocks((const void *)push_heavy_kernel);
-  J.gpush = push_resident;
-  J.gheavy = heavy_resident;
-  J.gcol = collect_grid(P.nwords, &ca.words);
+  if (is_large(P)) {
+    // its rounds reset their counters themselves
+    TSVD_CUDA(cudaMemsetAsync(P.counters + 1, 0, 3 * sizeof(int32_t), st));
+    pa.clock = ca.clock = reinterpret_cast<unsigned long long *>(P.counters + kCounters);
+    TSVD_CUDA(cudaMemsetAsync(pa.clock, 0, 2 * sizeof(unsigned long long), st));
+    ca.round = P.counters + 2;
+  }
+  J.gpush = grid_for((int64_t)1 << 30, 256, 8);
+  J.gcol = collect_grid(P);
   J.level = std::max(1, prm.levels) - 1;
   J.done = false;
   J.rounds = 0;
+  J.kernel_ms = 0;
   return TSVD_OK;
 }
 
@@ -686,14 +750,64 @@ float level_theta(const PprParams &prm, int level, float rmax_f) {
   return std::max(theta, rmax_f);
 }
 
+// Small graphs. A push here is a few dozen rounds of a few microseconds with all items
+// of a round side by side, and the pauses between separate launches are part of what
+// settles its state: launched as a graph, every run of the 4,000-vertex tenant ended in
+// one and the same state, as far from the middle of what separate launches give as
+// their own runs are, or twice as far.
+
+// Launches `count` rounds on the job's stream (asynchronous).
+tsvd_status job_rounds(PushJob &J, int count) {
+  PprState &P = *J.P;
+  cudaStream_t st = J.st;
+  for (int k = 0; k < count; ++k) {
+    const int cur = P.cur, nxt = 1 - P.cur;
+    J.pa.front = P.front[cur];
+    J.pa.front_count = P.counters + cur;
+    TSVD_CUDA(cudaMemsetAsync(P.counters + 2, 0, 2 * sizeof(int32_t), st));
+    TSVD_CUDA(cudaMemsetAsync(P.counters + nxt, 0, sizeof(int32_t), st));
+    TSVD_CUDA(cudaEventRecord(P.kev[2 * k], st));
+    push_kernel<false><<<J.gpush, 256, 0, st>>>(J.pa);
+    TSVD_LAUNCH_CHECK();
+    push_heavy_kernel<false><<<J.gpush, 256, 0, st>>>(J.pa);
+    TSVD_LAUNCH_CHECK();
+    TSVD_CUDA(cudaEventRecord(P.kev[2 * k + 1], st));
+    J.ca.next = P.front[nxt];
+    J.ca.next_count = P.counters + nxt;
+    collect_kernel<<<J.gcol, 256, 0, st>>>(J.ca);
+    TSVD_LAUNCH_CHECK();
+    P.cur = nxt;
+    ++J.rounds;
+  }
+  TSVD_CUDA(cudaMemcpyAsync(P.host_counters, P.counters, kCounters * sizeof(int32_t),
+                            cudaMemcpyDeviceToHost, st));
+  return TSVD_OK;
+}
+
+// Waits for the job's launched rounds; *empty: their frontier is.
+tsvd_status job_wait(PushJob &J, int count, const PprParams &prm, bool *empty) {
+  PprState &P = *J.P;
+  TSVD_CUDA(cudaStreamSynchronize(J.st));
+  for (int k = 0; k < count; ++k) {
+    float ms = 0.f;
+    if (cudaEventElapsedTime(&ms, P.kev[2 * k], P.kev[2 * k + 1]) == cudaSuccess) J.kernel_ms += ms;
+  }
+  if (P.host_counters[4]) return fail(TSVD_ERR_STATE, "push: frontier buffer overflow");
+  *empty = P.host_counters[P.cur] == 0;
+  if (!*empty && J.rounds >= prm.max_rounds)
+    return fail(TSVD_ERR_TIMEOUT, "push: %lld rounds without convergence", (long long)J.rounds);
+  return TSVD_OK;
+}
+
 }  // namespace
 
 constexpr int kRounds = 4;  // rounds launched together (even: the frontier lists end as they began)
 
-// The kernels of kRounds rounds as one graph launch: twelve separate launches
-// cost the host 60-120 us, more than the kernels of a small round. Its
+// Large graphs: the kernels of kRounds rounds as one graph launch. Twelve separate
+// launches cost the host 60-120 us, more than the kernels of a late round. Its
 // parameters are set again when a push has others (grown adjacency, next
-// threshold level).
+// threshold level). Steps, separate launches / this: 50k vertices pushed from scratch
+// 13.4 -> 12.5 ms, 100k 18.4 -> 17.8, 150k of degree 29 106.9 -> 104.3.
 struct RoundGraph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -725,9 +839,9 @@ struct RoundNode {
     ca.next = P.front[nxt];
     ca.next_count = P.counters + nxt;
     ca.spent = P.counters + cur;
-    const void *fn[3] = {(const void *)push_kernel, (const void *)push_heavy_kernel,
-                         (const void *)collect_kernel};
-    const int grid[3] = {J.gpush, J.gheavy, J.gcol};
+    const void *fn[3] = {(const void *)push_kernel<true>, (const void *)push_heavy_kernel<true>,
+                         (const void *)collect_large_kernel};
+    const int grid[3] = {J.gpush, J.gpush, J.gcol + 1};
     arg = k % 3 == 2 ? (void *)&ca : (void *)&pa;
     p.func = const_cast<void *>(fn[k % 3]);
     p.gridDim = dim3((unsigned)grid[k % 3]);
@@ -790,7 +904,7 @@ tsvd_status job_poll(PushJob &J, int slot, int64_t rounds, const PprParams &prm,
   TSVD_CUDA(cudaEventSynchronize(P.kev[slot]));
   const int32_t *h = P.host_counters + kCounters * slot;
   if (h[4]) return fail(TSVD_ERR_STATE, "push: frontier buffer overflow");
-  *empty = h[0] == 0 && h[kHighCount] == 0;
+  *empty = h[0] == 0;
   if (!*empty && rounds >= prm.max_rounds)
     return fail(TSVD_ERR_TIMEOUT, "push: %lld rounds without convergence", (long long)rounds);
   return TSVD_OK;
@@ -803,18 +917,18 @@ tsvd_status job_lower(PushJob &J, const PprParams &prm) {
   J.pa.theta_f = J.ca.theta_f = level_theta(prm, J.level, J.pa.rmax_f);
   unpark_kernel<<<grid_for(P.nwords, 256, 8), 256, 0, J.st>>>(P.tflag, P.pend, P.nwords);
   TSVD_LAUNCH_CHECK();
+  TSVD_CUDA(cudaMemsetAsync(P.counters + P.cur, 0, sizeof(int32_t), J.st));
   CollectArgs ca = J.ca;
-  ca.next = P.front[0];
-  ca.next_count = P.counters;
-  ca.spent = nullptr;
-  collect_kernel<<<J.gcol, 256, 0, J.st>>>(ca);
-  TSVD_LAUNCH_CHECK();
-  return TSVD_OK;
+  ca.next = P.front[P.cur];
+  ca.next_count = P.counters + P.cur;
+  return collect_launch(P, ca, J.st);
 }
 
 tsvd_status job_finish(PushJob &J, PushStats *out) {
   PprState &P = *J.P;
-  unsigned long long slots[kStatSlots * 4 + 2], hs[4] = {0, 0, 0, 0};
+  unsigned long long slots[kStatSlots * 4], hs[4] = {0, 0, 0, 0}, ns = 0;
+  if (J.pa.clock)
+    TSVD_CUDA(cudaMemcpyAsync(&ns, J.pa.clock + 1, sizeof ns, cudaMemcpyDeviceToHost, J.st));
   TSVD_CUDA(cudaMemcpyAsync(slots, P.stats, sizeof slots, cudaMemcpyDeviceToHost, J.st));
   TSVD_CUDA(cudaStreamSynchronize(J.st));
   for (int k = 0; k < kStatSlots * 4; ++k) hs[k % 4] += slots[k];
@@ -824,7 +938,7 @@ tsvd_status job_finish(PushJob &J, PushStats *out) {
     out->edge_updates = (int64_t)hs[1];
     out->items = (int64_t)hs[2];
     out->item_edges = (int64_t)hs[3];
-    out->kernel_ms = slots[kStatSlots * 4 + 1] * 1e-6;
+    out->kernel_ms = J.kernel_ms + ns * 1e-6;
   }
   P.seeded = false;
   return TSVD_OK;
@@ -837,19 +951,24 @@ tsvd_status ppr_push(PprState &P, const Adjacency &A, const PprParams &prm, uint
   PushJob J;
   TSVD_TRY(job_begin(J, P, A, prm, vmark, st));
   J.pa.theta_f = J.ca.theta_f = level_theta(prm, J.level, J.pa.rmax_f);
-  // The host looks at an interval's frontier while the next interval runs, so
-  // the GPU does not wait for it; rounds with an empty frontier cost 6 us each.
+  const int check_every = std::min(8, prm.check_every > 0 ? prm.check_every : 4);
   while (!J.done) {
-    TSVD_TRY(job_graph(J));
-    int slot = 0;
-    TSVD_TRY(job_interval(J, slot));
-    for (;;) {
-      TSVD_TRY(job_interval(J, 1 - slot));
-      J.rounds += kRounds;
-      bool empty = false;
-      TSVD_TRY(job_poll(J, slot, J.rounds, prm, &empty));
-      if (empty) break;
-      slot = 1 - slot;
+    bool empty = false;
+    if (is_large(P)) {
+      // The host looks at an interval's frontier while the next interval runs, so
+      // the GPU does not wait for it; rounds with an empty frontier cost 6 us each.
+      TSVD_TRY(job_graph(J));
+      TSVD_TRY(job_interval(J, 0));
+      for (int slot = 0; !empty; slot = 1 - slot) {
+        TSVD_TRY(job_interval(J, 1 - slot));
+        J.rounds += kRounds;
+        TSVD_TRY(job_poll(J, slot, J.rounds, prm, &empty));
+      }
+    } else {
+      while (!empty) {
+        TSVD_TRY(job_rounds(J, check_every));
+        TSVD_TRY(job_wait(J, check_every, prm, &empty));
+      }
     }
     if (J.level == 0)
       J.done = true;

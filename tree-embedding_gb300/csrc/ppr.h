@@ -14,19 +14,14 @@ __host__ __device__ __forceinline__ int64_t ppr_cell(int32_t v, int32_t s, int32
   return ((int64_t)(s >> 6) * n + v) * kChunk + (s & (kChunk - 1));
 }
 
-// A frontier list holds light items (degree <= kLightDegree) from its start and
-// the others from its end; the second count lies kHighCount after the first.
-// The light ones are pushed first, so that the costly vertices' residues, taken
-// last, hold what the round has sent them: neighbour reductions of a snapshot
-// 1994 M -> 1850 M (150k vertices of degree 29), 506 -> 449 M (300k of degree
-// 5) against one list; light up to 64: 1929 and 456 M, up to 1024: 1814 and 493 M.
-// In a graph of few pairs a round waits for latencies, not for reductions, and
-// one list does.
-constexpr int kLightDegree = 256;
-constexpr int64_t kLightPairs = 1 << 16;
-constexpr int kHighCount = 8;
-constexpr int kCounters = 16;
 constexpr int kStatSlots = 64;  // push counters are spread over this many slots
+constexpr int kCounters = 8;
+
+// (vertex, chunk) pairs from which a graph counts as large: its rounds are bound by
+// reductions and not by latencies, and it takes the kernels and launches made for that
+// (tested marks, collect_large_kernel, rounds launched as a graph). Below it these gain
+// little or move the results.
+constexpr int64_t kLargePairs = 1 << 16;
 
 struct RoundGraph;
 
@@ -39,6 +34,7 @@ struct PprState {
   int64_t nwords = 0;                // words of either bitset
   int2 *front[2] = {nullptr, nullptr};
   int64_t cap = 0;
+  int cur = 0;
   bool seeded = false;
   float *heavy_w = nullptr;
   int2 *heavy_item = nullptr;
@@ -47,9 +43,9 @@ struct PprState {
   int32_t *upd = nullptr;
   int32_t *counters = nullptr;
   int32_t *host_counters = nullptr;
-  unsigned long long *stats = nullptr;  // [kStatSlots][4], then a round's start and the
-                                        // scatter kernels' time so far (globaltimer, ns)
-  cudaEvent_t kev[2] = {};   // ends of the intervals in flight
+  unsigned long long *stats = nullptr;  // [kStatSlots][4]
+  cudaEvent_t kev[16] = {};  // scatter-kernel timing, two per round of a check interval; in
+                             // large graphs [0 .. 1] are the ends of the intervals in flight
   RoundGraph *graph = nullptr;  // the kernels of one interval (made by the first push)
 };
 
@@ -57,6 +53,7 @@ struct PprParams {
   double alpha = 0.2, rmax = 1e-7;
   int intdiv = 0;
   int undirected = 1;
+  int check_every = 4;
   int64_t max_rounds = 100000;
   int levels = 1;       // threshold schedule: rmax * ratio^(levels-1) ... rmax
   double ratio = 8.0;
@@ -71,9 +68,8 @@ struct PushStats {
 };
 
 struct PushArgs {
-  const int2 *front;           // light items from the start, the others from the end
-  const int32_t *front_count;  // [0] light, [kHighCount] the others
-  int64_t cap;
+  const int2 *front;
+  const int32_t *front_count;
   float *r, *p;
   const int64_t *off;
   const int32_t *deg, *nbr;
@@ -92,6 +88,7 @@ struct PushArgs {
   int32_t unit_cap;
   int32_t *overflow;
   unsigned long long *stats;
+  unsigned long long *clock;  // start of the round, scatter time so far (large graphs)
 };
 
 struct CollectArgs {
@@ -107,11 +104,9 @@ struct CollectArgs {
   int32_t *next_count;
   int64_t cap;
   int32_t *overflow;
-  int32_t light;    // items up to this degree are light (kLightDegree; all, in a small graph)
-  int words;        // bitset words per warp and step (1 .. 8)
   int32_t *spent;   // the round's own frontier count, reset here (null: not in a round)
   int32_t *round;   // counters[2 .. 3], reset for the next round
-  unsigned long long *clock;  // stats' last two entries
+  unsigned long long *clock;  // as in PushArgs
 };
 
 struct RefreshArgs {
