@@ -211,14 +211,15 @@ __global__ void __launch_bounds__(256) push_kernel(PushArgs a) {
       ok = __shfl_sync(kFull, ok, 0);
       slot = __shfl_sync(kFull, slot, 0);
       u0 = __shfl_sync(kFull, u0, 0);
-      const bool units_reserved = (int64_t)u0 + units <= a.unit_cap;
       if (ok) {
         reinterpret_cast<float2 *>(a.heavy_w)[(int64_t)slot * 32 + lane] = w;
         if (lane == 0) a.heavy_item[slot] = make_int2(v, c);
       }
-      if (units_reserved)
-        for (int32_t k = lane; k < units; k += 32)
-          a.units[u0 + k] = make_int2(ok ? slot : -1, k * kHeavy);
+      // push_heavy_kernel takes every unit below the count and the capacity, so those of
+      // a reservation without a slot, or that does not fit, are marked empty
+      const int32_t u1 = (int32_t)min((int64_t)u0 + units, (int64_t)a.unit_cap);
+      for (int32_t k = u0 + lane; k < u1; k += 32)
+        a.units[k] = make_int2(ok ? slot : -1, (k - u0) * kHeavy);
       if (ok) continue;
       // buffers full: process this hub inline
     }
