@@ -361,6 +361,7 @@ __global__ void __launch_bounds__(256) collect_large_kernel(CollectArgs a) {
     const int wk = lane >> 2;  // this lane's word and byte
     const bool mine = wbase + wk < a.nwords;
     const uint32_t word = mine ? __ldcg(a.tflag + wbase + wk) : 0u;
+    __syncwarp();  // four lanes read a word, one clears it
     if (word && gl == 0) a.tflag[wbase + wk] = 0;
     uint32_t byte = (word >> (8 * gl)) & 0xffu;
     int at = __popc(byte);
