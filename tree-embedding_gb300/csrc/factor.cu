@@ -19,6 +19,7 @@
 #include <cstdlib>
 
 #include "factor.h"
+#include "jacobi_sched.h"
 #include "philox_gauss.h"
 #include "plain.h"
 

@@ -167,13 +167,13 @@ size_t eig_work_bytes(int n, int nprob);
 // all n eigenvectors. refine = 1: g[b] = V^T G V for approximate eigenvectors V
 // (nearly diagonal); the diagonal is carried in fp64 (see jacobi_kernel) and
 // the rotations are replayed onto vinit[b] (V, n x n row-major), so v[b] = V R.
-// v may alias vinit.
+// v may alias vinit. *sweeps becomes kEigTimedOut (jacobi_sched.h) if a wait between
+// CTAs ran out.
 tsvd_status jacobi_eig_batched(double *const *g, int n, float *const *lambda,
                                float *const *v, int nprob, void *work,
                                size_t work_bytes, cudaStream_t st,
                                int32_t *sweeps, int refine = 0,
                                const float *const *vinit = nullptr);
 size_t jacobi_work_bytes(int n, int nprob);
-constexpr int32_t kEigTimedOut = 1 << 20;  // *sweeps if a wait between CTAs ran out
 
 }  // namespace tsvd

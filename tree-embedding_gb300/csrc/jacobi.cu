@@ -414,9 +414,10 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
     t = t1;
     sw = sw1;
   }
-  if (crank == 0 && threadIdx.x == 0) {
-    a.sweeps[prob] = sweeps_done;
-    atomicMax(a.most_sweeps, *dead ? kEigTimedOut : sweeps_done);
+  if (threadIdx.x == 0) {
+    if (crank == 0) a.sweeps[prob] = sweeps_done;
+    const int32_t report = jacobi_report(crank, *dead != 0, sweeps_done);
+    if (report) atomicMax(a.most_sweeps, report);
   }
   // eigenvalues to every CTA of the cluster, then each ranks its own players
   for (int i = threadIdx.x; i < 2 * nloc; i += blockDim.x) {

@@ -2,6 +2,7 @@
 // hand-over it implies when the pair slots are split over the CTAs of a
 // cluster. Host and device code: the host side is exercised by the CPU tests.
 #pragma once
+#include <stdint.h>
 
 #ifdef __CUDACC__
 #define TSVD_HD __host__ __device__ __forceinline__
@@ -65,6 +66,16 @@ TSVD_HD void circle_next(const int *top, const int *bot, int s0, int nloc, int P
     *nbot = nloc > 1 ? top[1] : dst_r;
   else
     *nbot = dst_l;
+}
+
+constexpr int32_t kEigTimedOut = 1 << 20;  // in place of a sweep count: a wait between CTAs ran out
+
+// What CTA `crank` of a solve's cluster reports; the solve's outcome is the largest of
+// its CTAs'. All of them count the same sweeps, but a wait runs out in one: it goes on
+// with values that did not come, and what it sends of them still completes the others'
+// waits, so each CTA speaks for itself.
+TSVD_HD int32_t jacobi_report(int crank, bool timed_out, int sweeps) {
+  return timed_out ? kEigTimedOut : crank == 0 ? sweeps : 0;
 }
 
 }  // namespace tsvd
