@@ -58,6 +58,7 @@ struct CallMemory {
 enum : uint32_t { kBadEntry = 1, kHasZeros = 2, kUnsorted = 4 };
 struct MatrixInfo {
   unsigned long long vmax_bits;  // largest magnitude, as the bits of a double
+  int64_t nnz;                   // entries that are not zero (sparse form)
   uint32_t found;
   int32_t nc;                    // columns that are not empty
 };
@@ -117,9 +118,10 @@ __global__ void check_kernel(RawMatrix m, int32_t *flag, int32_t *cnt, MatrixInf
   }
 }
 
-// cinv[c] = compacted column or -1 (in place of flag), cmap its inverse.
-__global__ void compact_kernel(int32_t *cinv, const int64_t *pos, int32_t ncols, int32_t *cmap,
-                               MatrixInfo *info) {
+// cinv[c] = compacted column or -1 (in place of flag), cmap its inverse. cpos: where
+// each column's nonzeros begin (may be null).
+__global__ void compact_kernel(int32_t *cinv, const int64_t *pos, const int64_t *cpos,
+                               int32_t ncols, int32_t *cmap, MatrixInfo *info) {
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncols;
        c += (int64_t)gridDim.x * blockDim.x) {
     const int32_t i = (int32_t)pos[c];
@@ -130,7 +132,10 @@ __global__ void compact_kernel(int32_t *cinv, const int64_t *pos, int32_t ncols,
       cinv[c] = -1;
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) info->nc = (int32_t)pos[ncols];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    info->nc = (int32_t)pos[ncols];
+    if (cpos) info->nnz = cpos[ncols];
+  }
 }
 
 __global__ void densify_kernel(RawMatrix m, const int32_t *cinv, double scale, int sp,
@@ -143,33 +148,58 @@ __global__ void densify_kernel(RawMatrix m, const int32_t *cinv, double scale, i
   }
 }
 
-// CSR of a matrix whose rows ascend and hold no zeros; (column, entry) pairs for
-// the sort that gives the CSC; column pointers of the compacted columns.
+// (column, entry) pairs for the sort that gives the CSC, zeros past the last column;
+// column pointers of the compacted columns; and, of a matrix whose rows ascend and hold
+// no zeros, the CSR.
 __global__ void csr_kernel(RawMatrix m, const int32_t *cinv, const int64_t *cpos, double scale,
-                           SparseBlock b, uint32_t *keys, uint32_t *vals) {
+                           bool ready, SparseBlock b, uint32_t *keys, uint32_t *vals) {
   const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   for (int64_t t = i0; t < m.nnz; t += step) {
-    const int32_t c = cinv[m.col[t] - m.base];
-    b.colidx[t] = c;
-    b.rval[t] = scaled(m.val[t], scale);
+    const double v = m.val[t];
+    const int32_t c = v == 0.0 ? b.cols : cinv[m.col[t] - m.base];
     keys[t] = (uint32_t)c;
     vals[t] = (uint32_t)t;
+    if (ready) {
+      b.colidx[t] = c;
+      b.rval[t] = scaled(v, scale);
+    }
   }
-  for (int64_t i = i0; i <= b.rows; i += step)
-    b.rowptr[i] = i < m.nrows ? m.rp[i] - m.org : m.nnz;
+  if (ready)
+    for (int64_t i = i0; i <= b.rows; i += step)
+      b.rowptr[i] = i < m.nrows ? m.rp[i] - m.org : m.nnz;
   for (int64_t c = i0; c <= m.ncols; c += step) {
-    if (c == m.ncols) b.colptr[b.cols] = m.nnz;
+    if (c == m.ncols) b.colptr[b.cols] = b.nnz;
     else if (cinv[c] >= 0) b.colptr[cinv[c]] = cpos[c];
   }
 }
 
-__global__ void csc_gather_kernel(RawMatrix m, const uint32_t *order, SparseBlock b) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < m.nnz;
+// rows receives each entry's row, the key of the sort back to rows; null if the CSR is
+// there already.
+__global__ void csc_gather_kernel(RawMatrix m, const uint32_t *order, double scale, SparseBlock b,
+                                  uint32_t *rows) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < b.nnz;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t t = order[i];
-    b.rowidx[i] = m.row_of(t);
-    b.cval[i] = b.rval[t];
+    const int32_t r = m.row_of(t);
+    b.rowidx[i] = r;
+    b.cval[i] = rows ? scaled(m.val[t], scale) : b.rval[t];
+    if (rows) rows[i] = (uint32_t)r;
+  }
+}
+
+// The CSR of entries sorted by row, in each row by column.
+__global__ void csr_gather_kernel(RawMatrix m, const int32_t *cinv, const uint32_t *order,
+                                  const uint32_t *row, double scale, SparseBlock b) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= b.nnz;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    // the rows that begin here: those past the entry before's, up to this one's
+    const int64_t last = i < b.nnz ? (int64_t)row[i] : b.rows;
+    for (int64_t r = i > 0 ? (int64_t)row[i - 1] + 1 : 0; r <= last; ++r) b.rowptr[r] = i;
+    if (i == b.nnz) break;
+    const int64_t t = order[i];
+    b.colidx[i] = cinv[m.col[t] - m.base];
+    b.rval[i] = scaled(m.val[t], scale);
   }
 }
 
@@ -292,8 +322,13 @@ tsvd_status take_sparse(DeviceArena &A, SparseBlock &sb, int rows, int cols, int
 
 // The block from the caller's arrays, on the device. *ready stays false where the
 // matrix is left to the host: an entry is not valid (the host's walk says which
-// comes first), or, for the sparse form, a row does not ascend, holds zeros or
-// the entries do not fit the sort's 32-bit positions.
+// comes first) or, for the sparse form, the entries do not fit the sort's 32-bit
+// positions. Of a sparse matrix whose rows do not ascend or hold zeros, the sort by
+// column drops the zeros and a second one by row gives the CSR: both are stable, so the
+// entries come in the order of the host's build. The whole call, k = 128, 1500 x 6000
+// with 900k entries, 10 % of them zeros, rows mixed, measured: 47 ms with the host's
+// build, 5.3 so (rows in order without zeros: 5.3); 600 x 3001 with 90k, k = 32: 4.6 and
+// 1.3 ms.
 tsvd_status block_on_device(CallMemory &M, int32_t nrows, int32_t ncols, int64_t nnz_arg,
                             const int64_t *row_ptr, const int32_t *col_idx, const double *values,
                             int32_t base, bool sparse, DirectBlock &D, bool *ready) {
@@ -340,11 +375,11 @@ tsvd_status block_on_device(CallMemory &M, int32_t nrows, int32_t ncols, int64_t
   }
   TSVD_TRY(scan_i32_to_i64(cinv, pos, ncols, tmp, st));
   if (sparse) TSVD_TRY(scan_i32_to_i64(cnt, cpos, ncols, tmp, st));
-  compact_kernel<<<grid_for(ncols, 256), 256, 0, st>>>(cinv, pos, ncols, cmap, info);
+  compact_kernel<<<grid_for(ncols, 256), 256, 0, st>>>(cinv, pos, cpos, ncols, cmap, info);
   TSVD_LAUNCH_CHECK();
   TSVD_CUDA(cudaMemcpyAsync(&h, info, sizeof h, cudaMemcpyDeviceToHost, st));
   TSVD_CUDA(cudaStreamSynchronize(st));
-  if ((h.found & kBadEntry) || (sparse && h.found)) return TSVD_OK;
+  if (h.found & kBadEntry) return TSVD_OK;
   D.nc = h.nc;
   D.cmap = cmap;
   D.cinv = cinv;
@@ -365,21 +400,38 @@ tsvd_status block_on_device(CallMemory &M, int32_t nrows, int32_t ncols, int64_t
     D.at = at;
     return TSVD_OK;
   }
+  const bool in_order = h.found == 0;
   uint32_t *keys, *vals, *keys2, *vals2;
   void *stmp;
   TSVD_TRY(M.carve([&](DeviceArena &A) -> tsvd_status {
-    TSVD_TRY(take_sparse(A, D.sb, sp, D.nc, nnz));
+    TSVD_TRY(take_sparse(A, D.sb, sp, D.nc, h.nnz));
     for (uint32_t **p : {&keys, &vals, &keys2, &vals2}) TSVD_TRY(device_take(&A, p, (size_t)nnz));
     return device_take(&A, (char **)&stmp, sort_tmp_bytes(nnz));
   }));
   csr_kernel<<<grid_for(std::max<int64_t>(nnz, ncols), 256), 256, 0, st>>>(
-      m, cinv, cpos, D.scale, D.sb, keys, vals);
+      m, cinv, cpos, D.scale, in_order, D.sb, keys, vals);
   TSVD_LAUNCH_CHECK();
-  int bits = 1;
-  while ((1ll << bits) < D.nc) ++bits;
+  // zeros have the key nc
+  auto bits_for = [](int64_t keys_up_to) {
+    int bits = 1;
+    while ((1ll << bits) <= keys_up_to) ++bits;
+    return bits;
+  };
   bool in_alt = false;
-  TSVD_TRY(stable_sort_pairs(keys, vals, keys2, vals2, nnz, bits, stmp, st, &in_alt));
-  csc_gather_kernel<<<grid_for(nnz, 256), 256, 0, st>>>(m, in_alt ? vals2 : vals, D.sb);
+  TSVD_TRY(stable_sort_pairs(keys, vals, keys2, vals2, nnz,
+                             bits_for(in_order ? D.nc - 1 : D.nc), stmp, st, &in_alt));
+  if (in_alt) {
+    std::swap(keys, keys2);
+    std::swap(vals, vals2);
+  }
+  csc_gather_kernel<<<grid_for(h.nnz, 256), 256, 0, st>>>(m, vals, D.scale, D.sb,
+                                                         in_order ? nullptr : keys);
+  TSVD_LAUNCH_CHECK();
+  if (in_order) return TSVD_OK;
+  TSVD_TRY(stable_sort_pairs(keys, vals, keys2, vals2, h.nnz, bits_for(nrows - 1), stmp, st,
+                             &in_alt));
+  csr_gather_kernel<<<grid_for(h.nnz + 1, 256), 256, 0, st>>>(
+      m, cinv, in_alt ? vals2 : vals, in_alt ? keys2 : keys, D.scale, D.sb);
   TSVD_LAUNCH_CHECK();
   return TSVD_OK;
 }
