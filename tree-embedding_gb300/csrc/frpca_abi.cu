@@ -516,20 +516,25 @@ tsvd_status frpca_direct(int32_t nrows, int32_t ncols, int64_t nnz, const int64_
       s1 = block_on_device(M, nrows, ncols, nnz, row_ptr, col_idx, values, index_base, sparse, D,
                            &ready);
   }
-  if (s1 != TSVD_OK || !ready) {
-    // the host's walk: its errors come before those of the device and of k and q
+  HostBlock H;
+  bool walked = false;
+  // The host's walk and, for the sparse form, its build in place of the device's: 16
+  // bytes an entry on the device, where the device's own build takes up to 44.
+  auto from_host = [&]() -> tsvd_status {
     cudaGetLastError();
-    HostBlock H;
-    TSVD_TRY(host_block(nrows, ncols, nnz, row_ptr, col_idx, values, index_base, H));
+    if (!walked)
+      TSVD_TRY(host_block(nrows, ncols, nnz, row_ptr, col_idx, values, index_base, H));
+    walked = true;
     if (!args_ok) return fail(TSVD_ERR_INVALID, "frpca: k=%d q=%d", k, q);
     D = DirectBlock();
-    if (!H.cmap.empty()) {
-      if (!M.st || !sparse) return s1 != TSVD_OK ? s1 : fail(TSVD_ERR_STATE, "frpca: matrix");
-      for (void *p : M.held) cudaFree(p);
-      M.held.clear();
-      TSVD_TRY(sparse_from_host(M, nrows, ncols, H, D));
-    }
-  }
+    if (H.cmap.empty()) return TSVD_OK;
+    if (!M.st || !sparse) return s1 != TSVD_OK ? s1 : fail(TSVD_ERR_STATE, "frpca: matrix");
+    for (void *p : M.held) cudaFree(p);
+    M.held.clear();
+    return sparse_from_host(M, nrows, ncols, H, D);
+  };
+  // its errors come before those of the device and of k and q
+  if (s1 != TSVD_OK || !ready) TSVD_TRY(from_host());
   if (D.nc == 0) {
     if (S) std::fill(S, S + k, 0.0);
     if (U) std::fill(U, U + (size_t)nrows * k, 0.0);
@@ -541,13 +546,22 @@ tsvd_status frpca_direct(int32_t nrows, int32_t ncols, int64_t nnz, const int64_
   float *du, *dv, *ds;
   double *stage;
   FrpcaWork W;
-  s1 = M.carve([&](DeviceArena &A) -> tsvd_status {
-    TSVD_TRY(device_take(&A, &du, (size_t)sp * k));
-    TSVD_TRY(device_take(&A, &dv, (size_t)D.nc * k));
-    TSVD_TRY(device_take(&A, &ds, (size_t)k));
-    TSVD_TRY(device_take(&A, &stage, (size_t)stage_n));
-    return frpca_work_alloc(W, 1, D.nc, sp, k + 5, k, true, &A, M.st);
-  });
+  auto take_work = [&]() {
+    return M.carve([&](DeviceArena &A) -> tsvd_status {
+      TSVD_TRY(device_take(&A, &du, (size_t)sp * k));
+      TSVD_TRY(device_take(&A, &dv, (size_t)D.nc * k));
+      TSVD_TRY(device_take(&A, &ds, (size_t)k));
+      TSVD_TRY(device_take(&A, &stage, (size_t)stage_n));
+      return frpca_work_alloc(W, 1, D.nc, sp, k + 5, k, true, &A, M.st);
+    });
+  };
+  s1 = take_work();
+  if (s1 == TSVD_ERR_OOM && sparse && !walked) {
+    // the call fits beside the 16 bytes an entry, but not beside what the build has left
+    frpca_work_free(W);
+    s1 = from_host();
+    if (s1 == TSVD_OK) s1 = take_work();
+  }
   if (s1 == TSVD_OK) {
     FrpcaProblem P;
     P.block = 0;
