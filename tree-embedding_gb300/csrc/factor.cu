@@ -352,10 +352,10 @@ static tsvd_status eig_refined(FrpcaWork &W, double *const *d_g, int n, float *c
 }
 
 // Eigenpairs of the Grams W.g (the nv leading eigenvectors): lam / v point into
-// W.lambda / W.v.
+// W.lambda / W.v. two_sided: by the solver of jacobi.cu.
 static tsvd_status eig_solve(FrpcaWork &W, double *const *d_g, int n, int nv, float *const *d_lam,
-                             float *const *d_v, int nprob, cudaStream_t st) {
-  if (W.direct && n > kDirectOneSided) return eig_refined(W, d_g, n, d_lam, d_v, nprob, st);
+                             float *const *d_v, int nprob, bool two_sided, cudaStream_t st) {
+  if (two_sided) return eig_refined(W, d_g, n, d_lam, d_v, nprob, st);
   return eig_gram_batched(d_g, n, nv, d_lam, d_v, nprob, W.eig_work, W.eig_bytes, W.eig_stat, st);
 }
 
@@ -495,7 +495,7 @@ tsvd_status frpca_batch(FrpcaWork &W, const FrpcaProblem *probs, int nprob, int 
   // eigSVD of Z = A^T Q (frpca.c:99-136): Gram, eigenpairs, top-d.
   TSVD_TRY(gram_batched((const float *const *)d_z, d_nc, max_nc, l, kLp, d_g, W.gram_work,
                         W.gram_bytes, nprob, st));
-  TSVD_TRY(eig_solve(W, d_g, l, d, d_lam, d_v, nprob, st));
+  TSVD_TRY(eig_solve(W, d_g, l, d, d_lam, d_v, nprob, W.direct, st));
   double *d_sum2 = W.sums;
   sigma_kernel<<<nprob, 128, 0, st>>>((const float *const *)d_lam, d, d_cs, d_csi, d_sout, d_sum2);
   TSVD_LAUNCH_CHECK();
@@ -530,7 +530,8 @@ namespace {
 // m[i] (|S| x n, ld n) -> Gram (compensated, fp64) -> eigenpairs ->
 // out = m V_d diag(f(s)), sigma_out = s (the d largest singular values).
 tsvd_status merge_finish(FrpcaWork &W, const MergeProblem *probs, int nprob, int n, int nsrc,
-                         int root_mode, const std::vector<float *> &m, cudaStream_t st) {
+                         int root_mode, const std::vector<float *> &m, bool two_sided,
+                         cudaStream_t st) {
   const int d = W.d;
   std::vector<float *> lam(nprob), v(nprob), cs(nprob), out(nprob), sout(nprob);
   std::vector<double *> g(nprob);
@@ -553,7 +554,7 @@ tsvd_status merge_finish(FrpcaWork &W, const MergeProblem *probs, int nprob, int
   TSVD_TRY(pk.upload(st));
   TSVD_TRY(gram_batched((const float *const *)d_m, d_rows, nsrc, n, n, d_g, W.gram_work,
                         W.gram_bytes, nprob, st));
-  TSVD_TRY(eig_solve(W, d_g, n, d, d_lam, d_v, nprob, st));
+  TSVD_TRY(eig_solve(W, d_g, n, d, d_lam, d_v, nprob, two_sided, st));
   merge_scale_kernel<<<nprob, 128, 0, st>>>((const float *const *)d_lam, d, root_mode, d_cs,
                                             d_sout);
   TSVD_LAUNCH_CHECK();
@@ -776,7 +777,7 @@ tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, 
   // Z = M V (|S| x p), problem i at W.z + i RK
   TSVD_TRY(sgemm_batched(false, nsrc, p, n, W.wm, n, sm, W.wv, p, sv, W.z, p, RK, nprob,
                          W.gram_work, W.gram_bytes, st));
-  return merge_finish(W, probs, nprob, p, nsrc, root_mode, z, st);
+  return merge_finish(W, probs, nprob, p, nsrc, root_mode, z, W.direct, st);
 }
 
 }  // namespace
@@ -792,7 +793,8 @@ tsvd_status merge_matrix(FrpcaWork &W, const float *m, int rows, int cols, float
     TSVD_CUDA(cudaMemcpyAsync(W.wm, m, sizeof(float) * rows * cols, cudaMemcpyDeviceToDevice, st));
     return merge_wide_core(W, &prob, 1, cols, rows, 0, st);
   }
-  return merge_finish(W, &prob, 1, cols, rows, 0, std::vector<float *>{const_cast<float *>(m)}, st);
+  return merge_finish(W, &prob, 1, cols, rows, 0, std::vector<float *>{const_cast<float *>(m)},
+                      W.direct, st);
 }
 
 tsvd_status merge_batch(FrpcaWork &W, const MergeProblem *probs, int nprob, int h, int nsrc,
@@ -820,7 +822,7 @@ tsvd_status merge_batch(FrpcaWork &W, const MergeProblem *probs, int nprob, int 
                                                                                    nsrc, d_m);
     TSVD_LAUNCH_CHECK();
   }
-  return merge_finish(W, probs, nprob, n, nsrc, root_mode, m, st);
+  return merge_finish(W, probs, nprob, n, nsrc, root_mode, m, W.direct, st);
 }
 
 tsvd_status lp_right_batch(FrpcaWork &W, const LpProblem *probs, int nprob, const float *u,

@@ -59,10 +59,6 @@ struct DeviceArena {
   bool count = false;
 };
 
-// Direct eigen-solves of up to this many columns take the one-sided solver:
-// there its results and the two-sided one's agree to 1e-5 (see jacobi.cu).
-constexpr int kDirectOneSided = 48;
-
 // arena: device buffers from it and staging from the heap, for a caller that
 // allocates once per call (frpca_work_free then frees the staging only);
 // otherwise every buffer on its own and pinned staging.

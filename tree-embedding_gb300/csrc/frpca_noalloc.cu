@@ -61,7 +61,6 @@ constexpr size_t kSumB = al(8);
 constexpr int64_t kGramChunks = (std::max(kNaMaxUsedCols, kNaMaxRows) + 127) / 128 + 1;
 constexpr size_t kGramB = al((size_t)kGramChunks * kNaMaxL * kNaMaxL * 8);
 constexpr size_t kJacB = al((size_t)30 * (kNaMaxL + 1) * ((kNaMaxL + 1) / 2) * 8) + 512 + al(kNaMaxL * 4);
-constexpr size_t kEigB = al((size_t)(kNaMaxL + 1) * ((kNaMaxL + 31) / 32 * 32) * 8 + kNaMaxL * 4 + 8);
 constexpr size_t kPtrSlots = 320;
 constexpr size_t kPtrB = al(kPtrSlots * 8);
 constexpr size_t kIntB = al(kPtrSlots * 4);
@@ -93,8 +92,7 @@ constexpr size_t kOffCs = kOffV + kVB;
 constexpr size_t kOffSum = kOffCs + kCsB;
 constexpr size_t kOffGram = kOffSum + kSumB;
 constexpr size_t kOffJac = kOffGram + kGramB;
-constexpr size_t kOffEig = kOffJac + kJacB;
-constexpr size_t kOffPtr = kOffEig + kEigB;
+constexpr size_t kOffPtr = kOffJac + kJacB;
 constexpr size_t kOffInt = kOffPtr + kPtrB;
 constexpr size_t kOffRowPtr = kOffInt + kIntB;
 constexpr size_t kOffCol = kOffRowPtr + kRowPtrB;
@@ -203,12 +201,10 @@ tsvd_status scratch_for_current_device(unsigned char **out) {
     // the fixed regions must hold what the shared kernels ask for at the limits
     const size_t gram_need = gram_work_bytes(std::max(kNaMaxUsedCols, kNaMaxRows), kNaMaxL, 1);
     const size_t jac_need = jacobi_work_bytes(kNaMaxL, 1);
-    const size_t eig_need = eig_work_bytes(kNaMaxL, 1);
-    if (gram_need > kGramB || jac_need > kJacB || eig_need > kEigB)
+    if (gram_need > kGramB || jac_need > kJacB)
       return fail(TSVD_ERR_STATE,
-                  "frpca_noalloc: static scratch too small for the kernels (Gram %zu > %zu, "
-                  "Jacobi %zu > %zu or eigen-solve %zu > %zu bytes)", gram_need, kGramB, jac_need,
-                  kJacB, eig_need, kEigB);
+                  "frpca_noalloc: static scratch too small for the kernels (Gram %zu > %zu or "
+                  "Jacobi %zu > %zu bytes)", gram_need, kGramB, jac_need, kJacB);
     void *p = nullptr;
     cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
     if (e != cudaSuccess || !p)
@@ -327,8 +323,6 @@ extern "C" tsvd_status tsvd_frpca_noalloc(int32_t nrows, int32_t ncols, int64_t 
     W.gram_bytes = kGramB;
     W.jac_work = base + kOffJac;
     W.jac_bytes = kJacB;
-    W.eig_work = base + kOffEig;
-    W.eig_bytes = kEigB;
     W.eig_stat = (int32_t *)(base + kOffMisc + 64);
     W.direct = true;
     W.dptr = (void **)(base + kOffPtr);

@@ -2,12 +2,15 @@
 // a thread-block cluster, replacing LAPACKE_dsyevd (Code/frpca.c:102) and the
 // Gram route to LAPACKE_dgesvd (..._mkl.c:1278).
 //
-// The sessions' eigen-solves and small direct ones use the one-sided solver of
-// eig.cu, which is faster and closer to the exact result. This one stays
-// behind the entry points that hand singular vectors to the caller
-// (tsvd_frpca*, tsvd_merge_svd) for more than kDirectOneSided columns: its
-// rotations shorten the vectors by up to 4e-5 at 256 columns, and callers who
-// keep results from earlier versions compare them at 2e-5.
+// The solver of the entry points that hand singular vectors to the caller
+// (tsvd_frpca*, tsvd_merge_svd); the sessions' eigen-solves take the one-sided solver of
+// eig.cu. The two differ in what they are good at. Its rotations shorten the vectors here, by 1e-6 (16 columns) to 4.4e-5
+// (256), where the one-sided solver's stay within 1e-6; but a vector's small entries
+// keep their relative accuracy here, and only an absolute one of 1e-7 there. Left
+// vectors are M V / s: of 300 x 16 with columns of norms 1 to 1e-6 they are orthogonal to
+// 3.5e-6 this way and to 3.2e-4 the other, which is what a caller of these entry points
+// sees. The tree works on its factors' products, and the root's is off by 0.9e-6 (d = 16)
+// to 1.8e-5 (128) by this solver and by 2.0e-6 to 6.4e-6 by the other.
 #include <algorithm>
 
 #include <cooperative_groups.h>
@@ -177,6 +180,19 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
   const int s0 = crank * L, nloc = min(P, s0 + L) - s0;  // >= 1 (host)
   const int cgroups = (int)blockDim.x / P;  // >= 8 (P <= 128)
   const double *Gin = a.g[prob];
+  // G times a power of two, its largest diagonal entry in [1, 2): the products of two
+  // entries in the rotations' tests stay in range, and nothing else changes
+  double down, up;
+  {
+    long long big = 0;
+    for (int i = threadIdx.x & 31; i < n; i += 32)
+      big = max(big, __double_as_longlong(fabs(Gin[(int64_t)i * n + i])));
+    for (int o = 16; o > 0; o >>= 1) big = max(big, __shfl_xor_sync(0xffffffffu, big, o));
+    const int raw = (int)(big >> 52);  // 0: zero or denormal, 0x7ff: not finite
+    const int e = raw > 0 && raw < 0x7ff ? raw - 1023 : 0;
+    down = scalbn(1.0, -e);
+    up = scalbn(1.0, e);
+  }
   float2 *log = a.log + (int64_t)prob * JAC_MAX_SWEEPS * (np - 1) * P;
   // at every sweep start slot k holds players k (top) and np-1-k (bottom)
   auto player_of = [&](int i) { return (i & 1) ? np - 1 - (s0 + i / 2) : s0 + i / 2; };
@@ -187,12 +203,12 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
     slot_m[i] = slot_m[L + i] = make_int2(2 * i * np, (2 * i + 1) * np);
   }
   for (int i = threadIdx.x; i < np; i += blockDim.x) {
-    dbase[i] = (refine && i < n) ? Gin[(int64_t)i * n + i] : 0.0;
-    diag[i] = (!refine && i < n) ? (float)Gin[(int64_t)i * n + i] : 0.f;
+    dbase[i] = (refine && i < n) ? Gin[(int64_t)i * n + i] * down : 0.0;
+    diag[i] = (!refine && i < n) ? (float)(Gin[(int64_t)i * n + i] * down) : 0.f;
   }
   for (int k = threadIdx.x; k < P; k += blockDim.x) {  // round 0 pairs (k, np-1-k)
     const int q = np - 1 - k;
-    coup[k] = q < n ? (float)Gin[(int64_t)k * n + q] : 0.f;
+    coup[k] = q < n ? (float)(Gin[(int64_t)k * n + q] * down) : 0.f;
   }
   for (int i = threadIdx.x; i <= JAC_MAX_SWEEPS + 1; i += blockDim.x) flag[i] = 0;
   volatile int *dead = flag + JAC_MAX_SWEEPS + 1;  // a wait ran out
@@ -205,7 +221,7 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
   for (int idx = threadIdx.x; idx < 2 * nloc * np; idx += blockDim.x) {
     const int b = idx / np, col = idx % np, x = player_of(b);
     float v = 0.f;
-    if (x < n && col < n && !(refine && x == col)) v = (float)Gin[(int64_t)x * n + col];
+    if (x < n && col < n && !(refine && x == col)) v = (float)(Gin[(int64_t)x * n + col] * down);
     rows[(size_t)b * np + col] = v;
   }
   if (C > 1) cluster.sync(); else __syncthreads();
@@ -437,7 +453,7 @@ __global__ void __launch_bounds__(JAC_THREADS) jacobi_kernel(JacobiArgs a) {
       r += (lj > li) || (lj == li && j < x);
     }
     a.rank[prob * n + x] = r;
-    lam[r] = (float)li;
+    lam[r] = (float)(li * up);
   }
 }
 
