@@ -777,7 +777,7 @@ tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, 
   // Z = M V (|S| x p), problem i at W.z + i RK
   TSVD_TRY(sgemm_batched(false, nsrc, p, n, W.wm, n, sm, W.wv, p, sv, W.z, p, RK, nprob,
                          W.gram_work, W.gram_bytes, st));
-  return merge_finish(W, probs, nprob, p, nsrc, root_mode, z, W.direct, st);
+  return merge_finish(W, probs, nprob, p, nsrc, root_mode, z, false, st);
 }
 
 }  // namespace

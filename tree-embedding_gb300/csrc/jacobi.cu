@@ -2,9 +2,10 @@
 // a thread-block cluster, replacing LAPACKE_dsyevd (Code/frpca.c:102) and the
 // Gram route to LAPACKE_dgesvd (..._mkl.c:1278).
 //
-// The solver of the entry points that hand singular vectors to the caller
-// (tsvd_frpca*, tsvd_merge_svd); the sessions' eigen-solves take the one-sided solver of
-// eig.cu. The two differ in what they are good at. Its rotations shorten the vectors here, by 1e-6 (16 columns) to 4.4e-5
+// The solver of the entry points that hand singular vectors of a matrix of up to 256
+// columns to the caller (tsvd_frpca*, tsvd_merge_svd); the sessions' eigen-solves, and
+// the end of a wider merge, take the one-sided solver of eig.cu. The two differ in what
+// they are good at. Its rotations shorten the vectors here, by 1e-6 (16 columns) to 4.4e-5
 // (256), where the one-sided solver's stay within 1e-6; but a vector's small entries
 // keep their relative accuracy here, and only an absolute one of 1e-7 there. Left
 // vectors are M V / s: of 300 x 16 with columns of norms 1 to 1e-6 they are orthogonal to
