@@ -344,15 +344,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_kernel(GemmArgs a) 
 }
 
 // ------------------------------------------------------------------ Gram
-// Sums of products in pairs of floats. The rows are taken GRAM_SUB at a time;
-// over them column i has norm at most pw_i (a power of two), so a partial sum of
-// x_i x_j stays within pw_i pw_j and s = 3 pw_i pw_j + sum keeps one exponent:
-// what a fused multiply-add rounds away is then exactly the product minus the
-// change of s, and a second one recovers it for c (to 2^-47 of pw_i pw_j): four
-// operations a term, where the error-free product and TwoSum of any two floats
-// (Ogita, Rump, Oishi, SISC 2005) take ten. The sub-blocks' sums are added to
-// (S, C) by TwoSum, and the chunks in fp64. The kernel is bound by the issue of
-// these operations; 32 problems of 1500 x 256, measured: 463 -> 297 us.
+// Compensated sums of error-free products (Ogita, Rump, Oishi, "Accurate sum and dot
+// product", SISC 2005): S + C carries a chunk's sum to 2^-45 of the sum of its
+// terms' magnitudes, and the chunks are added in fp64. Of TwoSum's error of u = S + p,
+// (S - S') + (p - z) with z = u - S and S' = u - z, the second difference is taken of the
+// exact product instead of p, by one fused multiply-add: eight operations a term, where
+// p's own error and TwoSum take ten. (u itself from the exact product would take seven,
+// but u - z then rounds where S and the product cancel: 2^-28. Four are enough with S held
+// near an anchor above the column norms, but entries then carry 2^-45 of the norms'
+// product, and those of nearly orthogonal columns 2^-30 of their terms.) The kernel is
+// bound by the issue of these operations; with the sum of the chunks, measured, 32
+// problems of 1500 x 256: ten 996 us, these 652, anchored 583; 64 of 3125 x 133: 1084,
+// 732, 643.
 constexpr int GRAM_MIN_ROWS = 128;    // rows per CTA (one fp64 partial per chunk); fewer
                                       // where CTAs are few (gram_batched)
 constexpr int GRAM_MAX_CHUNKS = 2048;  // chunks over all problems (bounds the work buffer)
@@ -371,23 +374,22 @@ struct GramArgs {
   double *work;   // [prob][chunk][l*l]
 };
 
-// The least power of two above sqrt(sum) (0 for 0), at most 2^62: three times its
-// square is still a float (beyond it the pair only rounds as plain sums do).
-__device__ __forceinline__ float norm_bound(float sum) {
-  const int e = min((int)(__float_as_uint(sum) >> 23) - 127, 123);
-  return sum > 0.f ? __uint_as_float((uint32_t)((e >> 1) + 1 + 127) << 23) : sum;
+// (S, C) += a b
+__device__ __forceinline__ void comp_add(float &S, float &C, float a, float b) {
+  const float u = __fadd_rn(S, __fmul_rn(a, b)), z = __fsub_rn(u, S);
+  C = __fadd_rn(C, __fadd_rn(__fsub_rn(S, __fsub_rn(u, z)), __fmaf_rn(a, b, -z)));
+  S = u;
 }
 
 // grid: (row chunk, tile group, problem). A thread owns one upper-triangle 4 x 4
 // tile of the l x l output and accumulates it over the chunk's rows.
 __global__ void __launch_bounds__(GRAM_THREADS) gram_partial_kernel(GramArgs a) {
-  extern __shared__ __align__(16) float sx[];  // [GRAM_SUB][4 tiles], then [4 tiles] bounds
+  extern __shared__ __align__(16) float sx[];  // [GRAM_SUB][4 tiles]
   const int prob = blockIdx.z, chunk = blockIdx.x;
   const int rows = a.rows[prob];
   const int r0 = chunk * a.chunk_rows;
   double *out = a.work + ((int64_t)prob * a.nchunks + chunk) * a.l * a.l;
   const int T = a.tiles, sld = 4 * T;  // staged row stride covers every 4 x 4 tile column
-  float *pw = sx + GRAM_SUB * sld;
   const float *x = a.x[prob];
   const int r1 = min(rows, r0 + a.chunk_rows);
   const int t = blockIdx.y * GRAM_THREADS + threadIdx.x;
@@ -411,41 +413,14 @@ __global__ void __launch_bounds__(GRAM_THREADS) gram_partial_kernel(GramArgs a) 
       sx[i] = (rr < nr && cc < a.l) ? x[(int64_t)(rb + rr) * a.ld + cc] : 0.f;
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < sld; c += GRAM_THREADS) {
-      float sum = 0.f;
-#pragma unroll 8
-      for (int rr = 0; rr < GRAM_SUB; ++rr) sum = fmaf(sx[rr * sld + c], sx[rr * sld + c], sum);
-      pw[c] = norm_bound(sum);
-    }
-    __syncthreads();
     if (!mine) continue;
-    float pi[4], pj[4], s[16], c[16];
-    *reinterpret_cast<float4 *>(pi) = *reinterpret_cast<const float4 *>(pw + ti);
-    *reinterpret_cast<float4 *>(pj) = *reinterpret_cast<const float4 *>(pw + tj);
-#pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      s[e] = 3.f * (pi[e >> 2] * pj[e & 3]);
-      c[e] = 0.f;
-    }
 #pragma unroll 2
     for (int rr = 0; rr < nr; ++rr) {
       float xi[4], xj[4];
       *reinterpret_cast<float4 *>(xi) = *reinterpret_cast<const float4 *>(sx + rr * sld + ti);
       *reinterpret_cast<float4 *>(xj) = *reinterpret_cast<const float4 *>(sx + rr * sld + tj);
 #pragma unroll
-      for (int e = 0; e < 16; ++e) {
-        const float u = __fmaf_rn(xi[e >> 2], xj[e & 3], s[e]);
-        const float z = __fsub_rn(u, s[e]);
-        c[e] = __fadd_rn(c[e], __fmaf_rn(xi[e >> 2], xj[e & 3], -z));
-        s[e] = u;
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < 16; ++e) {
-      const float v = __fsub_rn(s[e], 3.f * (pi[e >> 2] * pj[e & 3]));
-      const float u = __fadd_rn(S[e], v), z = __fsub_rn(u, S[e]);
-      C[e] += __fadd_rn(__fsub_rn(S[e], __fsub_rn(u, z)), __fsub_rn(v, z)) + c[e];
-      S[e] = u;
+      for (int e = 0; e < 16; ++e) comp_add(S[e], C[e], xi[e >> 2], xj[e & 3]);
     }
   }
   if (!mine) return;
@@ -842,7 +817,7 @@ tsvd_status gram_batched(const float *const *x, const int32_t *rows, int max_row
     chunk_rows = cr;
     nchunks = (int)nc;
   }
-  size_t smem = (size_t)(GRAM_SUB + 1) * (4 * tiles) * sizeof(float);
+  size_t smem = (size_t)GRAM_SUB * (4 * tiles) * sizeof(float);
   TSVD_TRY(raise_smem_ceiling((const void *)gram_partial_kernel, smem));
   // (a chunk past a problem's row count writes zeros)
   GramArgs a{x, rows, ld, l, tiles, nchunks, chunk_rows, work};
