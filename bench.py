@@ -707,8 +707,7 @@ def main():
             "sparse_blocks_mean": float(np.mean([s["sparse_blocks"] for s in res["stages"]])),
             "autotuner_density": float(res["stages"][-1]["tune_density"]),
             "eig_sweeps_merge_max": int(max(s["eig_sweeps_merge"] for s in res["stages"])),
-            "merge_subspace_iters_max": int(max(s["merge_subspace_iters"] for s in res["stages"])),
-            "eig_refine_sweeps_max": int(max(s["eig_refine_sweeps"] for s in res["stages"]))}
+            "merge_subspace_iters_max": int(max(s["merge_subspace_iters"] for s in res["stages"]))}
     line["roofline"] = push_roofline(res["stages"])
     line["tail"] = tail_attribution(res["stages"])
     if "e2e_ms" in res:

@@ -609,21 +609,6 @@ __global__ void trace_kernel(const float *__restrict__ k, int l, double *__restr
   if (threadIdx.x == 0) out[blockIdx.x] = acc;
 }
 
-__global__ void diag_sum_kernel(double *const *g, int l, double *out) {
-  const int prob = blockIdx.x;
-  double acc = 0.0;
-  for (int i = threadIdx.x; i < l; i += blockDim.x) acc += g[prob][(int64_t)i * l + i];
-  __shared__ double red[256];
-  red[threadIdx.x] = acc;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[prob] = red[0];
-}
-
-
 constexpr int64_t kWideK = 256 * 256 + 256 * 288;  // fp32 Gram + chol_factor_floats(256)
 
 // Buffers for up to `nprob` problems of n columns and W.sp rows.
@@ -648,10 +633,9 @@ tsvd_status wide_reserve(FrpcaWork &W, int nprob, int n) {
   return TSVD_OK;
 }
 
-// x[i] (rows x p, ld p) -> x[i] R^-1 into y[i], R from the compensated Gram;
-// energy (optional, host, nprob) receives trace(x^T x) = ||x||_F^2 per problem.
+// x[i] (rows x p, ld p) -> x[i] R^-1 into y[i], R from the compensated Gram.
 tsvd_status orthonormalize(FrpcaWork &W, float *x, int64_t xstride, float *y, int rows, int p,
-                           int nprob, cudaStream_t st, double *energy) {
+                           int nprob, cudaStream_t st) {
   std::vector<float *> xs(nprob);
   std::vector<double *> g(nprob);
   std::vector<int32_t> rr(nprob, rows);
@@ -667,11 +651,6 @@ tsvd_status orthonormalize(FrpcaWork &W, float *x, int64_t xstride, float *y, in
   TSVD_TRY(pk.upload(st));
   TSVD_TRY(gram_batched((const float *const *)d_x, d_rows, rows, p, p, d_g, W.gram_work,
                         W.gram_bytes, nprob, st));
-  if (energy) {
-    diag_sum_kernel<<<nprob, 256, 0, st>>>(d_g, p, W.sums);
-    TSVD_LAUNCH_CHECK();
-    TSVD_CUDA(cudaMemcpyAsync(energy, W.sums, sizeof(double) * nprob, cudaMemcpyDeviceToHost, st));
-  }
   TSVD_TRY(orth_gram_batched(d_g, p, x, y, rows, xstride, nprob, W.eig_work, W.eig_bytes, st));
   TSVD_CUDA(cudaStreamSynchronize(st));
   return TSVD_OK;
@@ -680,12 +659,12 @@ tsvd_status orthonormalize(FrpcaWork &W, float *x, int64_t xstride, float *y, in
 // Merge of h * d > 256 columns. The top-d singular triplets of M = [B_1..B_h]
 // (|S| x n) come from a p = min(256, n, |S|) dimensional basis V of M's
 // dominant right singular subspace, found by subspace iteration
-// (Y = M V, W = M^T Y, each product re-orthonormalized by CholeskyQR on a
-// compensated Gram), started from the p columns of M with the largest norms
-// and stopped when ||M V||_F^2 gains less than 1e-7 of itself. The result is
-// then the merge of the p columns of M V (compensated Gram + eigen-solve), the
-// same arithmetic as a narrow merge. The products are plain fp32 GEMMs
-// (sgemm_batched: fixed-order sums).
+// (Y = M V, W = M^T Y), started from the p columns of M with the largest norms and
+// stopped when ||M V||_F^2 gains less than 1e-6 of itself. After each product a
+// well-conditioned basis is enough (fp32 Gram, shifted Cholesky); the last one is made
+// orthonormal from a compensated Gram. The result is then the merge of the p columns of
+// M V (compensated Gram + one-sided eigen-solve), as for a session's narrow merge. The
+// products are plain fp32 GEMMs (sgemm_batched: fixed-order sums).
 tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, int n, int nsrc,
                             int root_mode, cudaStream_t st);
 
@@ -768,7 +747,7 @@ tsvd_status merge_wide_core(FrpcaWork &W, const MergeProblem *probs, int nprob, 
   }
   // one accurate CholeskyQR pass: an orthonormal V to working precision
   TSVD_CUDA(cudaMemcpyAsync(W.ww, W.wv, sizeof(float) * nprob * sv, cudaMemcpyDeviceToDevice, st));
-  TSVD_TRY(orthonormalize(W, W.ww, sv, W.wv, n, p, nprob, st, nullptr));
+  TSVD_TRY(orthonormalize(W, W.ww, sv, W.wv, n, p, nprob, st));
   W.wide_iters = it + 1;
   // Rayleigh-Ritz: the narrow merge of the p columns of Z = M V
   const int64_t RK = std::max<int64_t>(W.rows_max * kLp, (int64_t)W.sp * 256);
