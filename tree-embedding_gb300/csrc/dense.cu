@@ -359,6 +359,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) umma_gemm_kernel(GemmArgs a) 
 constexpr int GRAM_MIN_ROWS = 128;    // rows per CTA (one fp64 partial per chunk); fewer
                                       // where CTAs are few (gram_batched)
 constexpr int GRAM_MAX_CHUNKS = 2048;  // chunks over all problems (bounds the work buffer)
+constexpr int GRAM_HALVED = 64;   // chunks of a problem that halving may make
 constexpr int GRAM_SUB = 32;      // rows staged in smem at a time
 constexpr int GRAM_THREADS = 256;
 constexpr int GRAM_LMAX = 256;
@@ -806,12 +807,14 @@ tsvd_status gram_batched(const float *const *x, const int32_t *rows, int max_row
   int tiles = (l + 3) / 4;
   int groups = (int)ceil_div(tiles * (tiles + 1) / 2, GRAM_THREADS);
   // A slab of 32 rows is 3 us of a CTA's issue: halve the chunks until every SM has
-  // two, as far as the buffer goes (with the sum of the chunks, 1000 x 69, 4
-  // problems: 18 -> 11 us; 6000 x 133, one: 38 -> 30 us).
+  // two, as far as the buffer goes and to GRAM_HALVED of a problem at most, as their sum
+  // is a chain. With it, chunks of 128 rows / halved / halved without that limit: 1000 x
+  // 69, 4 problems 35 / 20 / 20 us; one of 1500 x 256 47 / 42 / 42, 3000 x 133 43 / 33 /
+  // 39, 6000 x 133 47 / 47 / 60, 3000 x 69 37 / 31 / 29; two of 6000 x 37 31 / 31 / 39.
   while (chunk_rows > GRAM_SUB && (int64_t)nchunks * groups * nprob < 2 * sm_count()) {
     const int cr = (int)round_up(chunk_rows / 2, GRAM_SUB);
     const int64_t nc = ceil_div(max_rows, cr);
-    if (cr == chunk_rows || nc * nprob > GRAM_MAX_CHUNKS ||
+    if (cr == chunk_rows || nc > GRAM_HALVED || nc * nprob > GRAM_MAX_CHUNKS ||
         (size_t)(nc * nprob) * l * l * sizeof(double) > work_bytes)
       break;
     chunk_rows = cr;
