@@ -83,7 +83,7 @@ typedef struct {
  * tsvd_set_frpca_seed() (the reference seeds MKL VSL with time(NULL)). The
  * caller's double values are rounded to float and both products run as FP32
  * SpMM on the GPU (tsvd_frpca_fp32); the small solves are fp32 with fp64
- * Grams and an accurate eigen-solve, so results match the reference's
+ * Grams and an fp64-refined eigen-solve, so results match the reference's
  * FP64 frPCA to about 1e-6 relative in the leading singular values, not to
  * double precision.
  * Errors are reported through tsvd_last_error(); the legacy signature has no

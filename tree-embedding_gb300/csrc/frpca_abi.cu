@@ -8,8 +8,8 @@
 // the legacy frPCA symbol; both products as SpMM, the plain form's products).
 // Built on one host thread instead, with some 40 allocations a call, this and
 // the results' transposition were most of a call. 1500 x 6000 with 900k entries,
-// k = 128, measured: 12.7 -> 6.3 ms; 600 x 3001 with 90k entries, k = 32: 3.9 ->
-// 1.8 ms.
+// k = 128, measured with the kernels of then: 12.7 -> 6.3 ms (5.6 now); 600 x 3001 with
+// 90k entries, k = 32: 3.9 -> 1.8 ms (1.8 now).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
